@@ -842,6 +842,7 @@ flb_status streams_setup(flb_batch b, int nstreams) {
       if (s != FLB_OK) return bfail(b, s, flb_last_error(b->handles[c]));
     }
   }
+  for (flb_handle h : b->handles) set_peers(h, std::min(b->n, (uint32_t)nstreams));
   b->nstreams = nstreams;
   return FLB_OK;
 }

@@ -57,6 +57,7 @@ struct KParams {
   // 1-w, -3k, F/2, F (zero without forcing), and per direction pair q (odd
   // direction 2q+1) 3k c.F and 9k c.F, with k = 1 - w/2
   float fu_omc, fu_nk3, fu_hfx, fu_hfy, fu_fx, fu_fy;
+  float fu_nhfx, fu_nhfy;  // -F/2
   float fu_g[4], fu_h[4];
   float fu_sw[3];  // FP16S deviation form: f16_scale * w for directions 0, 1..4, 5..8
   int has_io;      // the case has inlet or outlet cells
@@ -156,6 +157,20 @@ __device__ __forceinline__ void clear_next_lists(const ListClear& lc) {
   if (threadIdx.x < 2) lc.counts[threadIdx.x] = 0u;
   for (uint32_t i = threadIdx.x; i < lc.nwords; i += blockDim.x) lc.bits[i] = 0u;
 }
+
+// A launch of several single-phase steps (k_mt.cu): T steps from t, on windows
+// of W x H cells of which OW x OH are output; columns start pad cells left of
+// the output.  The state is read through KParams and written to dst.
+struct MtArgs {
+  void* dst;
+  uint32_t t;
+  int T, W, H, OW, OH, pad;
+  int bx, tiles;  // windows per row of windows, and in all
+  int vec;      // rows move in groups of four cells (nx % 4 == 0)
+  int wm;       // the last step writes density and velocity
+  int threads;
+  int pairs;    // FP32 fused: two cells per thread with packed arithmetic
+};
 
 // What the persistent free-surface step (k_fsp.cu) needs besides the step
 // parameters: the lists and their lengths of both parities (read by the step

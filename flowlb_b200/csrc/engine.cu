@@ -16,6 +16,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "../../include/flowlb.h"
@@ -42,6 +44,7 @@ struct GraphSlot {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   uint64_t kernels = 0;
+  const void* f = nullptr;  // population buffer it was captured with
 };
 
 }  // namespace
@@ -93,6 +96,12 @@ struct flb_engine {
   KParams kp{};
   // device buffers
   void* d_f = nullptr;
+  // single phase: the second population buffer of the multi-step kernel (d_f is
+  // the current one); null: one step per launch
+  void* d_f2 = nullptr;
+  // handles stepped concurrently with this one (the batch's streams form): the
+  // windows are sized for them together, and the launches come from graphs
+  uint32_t peers = 1;
   void* d_rho = nullptr;
   void* d_u = nullptr;
   uint8_t* d_flags[2] = {nullptr, nullptr};
@@ -111,6 +120,7 @@ struct flb_engine {
   uint32_t* d_tstep = nullptr;  // [2] time step by parity (FP16S stochastic rounding)
   uint32_t* d_plain = nullptr;  // single phase: plain-fluid chunk map (k_plain_chunks)
   GraphSlot g_pair, g_big;
+  GraphSlot g_mt[4];  // multi-step launches, by step parity and by which buffer is current
   std::string err;
 };
 
@@ -168,6 +178,11 @@ struct Ops {
     h->grid_sc = (uint32_t)(nsm * sc_list_blocks_per_sm<S, C, M>(h->use_vec_list));
     h->grid_fs1 = (uint32_t)(nsm * fs_blocks_per_sm<S, C, M>(0, 0));
     h->grid_fs234 = (uint32_t)(nsm * fs_blocks_per_sm<S, C, M>(1, h->fs_form));
+  }
+  static cudaError_t mt(flb_engine* h, const MtArgs& a) {
+    if constexpr (std::is_same<S, float>::value && std::is_same<M, float>::value)
+      return launch_mt<S, C, double>(h->kp, a, h->stream, h->fused);  // the mass type is not used here
+    else return launch_mt<S, C, M>(h->kp, a, h->stream, h->fused);
   }
   static void apply_recon(flb_engine* h, uint32_t odd) { launch_apply_recon<S, C, M>(h->kp, h->stream, odd); }
   static cudaError_t persist(flb_engine* h, const KParams& p0, const KParams& p1, const FspArgs& a) {
@@ -351,7 +366,8 @@ void destroy_graph(GraphSlot& g) {
 // Captures 2*pairs steps starting at an even t with flag buffer 0 current:
 // the passes of every step, or one persistent launch (free surface, h->persist).
 flb_status capture(flb_engine* h, GraphSlot& g, int pairs) {
-  if (g.exec) return FLB_OK;
+  if (g.exec && g.f == h->d_f) return FLB_OK;
+  destroy_graph(g);
   const int saved_cur = h->cur;
   FLB_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   uint64_t kernels = 0;
@@ -382,6 +398,151 @@ flb_status capture(flb_engine* h, GraphSlot& g, int pairs) {
   g.graph = graph;
   g.exec = exec;
   g.kernels = kernels;
+  g.f = h->d_f;
+  return FLB_OK;
+}
+
+// ---- single phase: several steps per launch (k_mt.cu) -----------------------
+// The window sizes a grid may use: steps per launch, window columns and rows,
+// threads, and packed pairs or one cell per thread.  On small grids the launch
+// is one round of windows and its latency is what counts, so the windows are
+// small (more of them, more recomputed cells) and take many steps; on large
+// grids the recomputed cells count, so the windows are as large as still lets
+// three (FP64: two) run per SM.  Measured on a B200 in us per step, old = one
+// step per launch (grid, storage: old | small windows ... large ones):
+//   256x64    F32 4.1 | 8 x 32x24: 1.05    4 x 32x24: 1.5     4 x 64x22: 2.2
+//   512x160   F32 4.0 | 2.8                1.79               6 x 64x32: 2.2   4 x 64x22: 2.2
+//   1024x256  F32 4.6 | 6.9                3.9                2.9              3.9
+//   1400x360  F32 8.7 | 12.8               6.7                5.1              4.9
+//   4096x1024 F32 50  | 106                52                 34               28.5
+//   1025x256  F64 8.5 | 14                 7.9                5.2              6.2
+//   4097x1024 F64 114 | 231                123                73               66
+//   1025x256  F16 5.6 | 16                 7.9                4.9              5.2
+//   4096x1024 F16 27  | 243                111                53               42
+// FP16 storage above 300,000 cells and FP32 with the reference arithmetic above
+// 110,000 (1024x256: 5.8 | 5.5; 2048x512: 15.8 | 17.1) stay at one step per launch.
+struct MtWindow {
+  uint64_t cells;  // for grids of up to this many cells
+  int T, W, H, threads, pairs;
+};
+constexpr uint64_t kAnyCells = ~0ull;
+constexpr MtWindow kMtF32[] = {{18000, 8, 32, 24, 384, 1}, {110000, 4, 32, 24, 384, 1}, {400000, 6, 64, 32, 512, 1},
+                               {kAnyCells, 4, 64, 22, 256, 1}};
+constexpr MtWindow kMtF32Ref[] = {{25000, 8, 32, 24, 384, 0}, {75000, 4, 32, 24, 384, 0}, {110000, 6, 64, 28, 896, 0}};
+constexpr MtWindow kMtF64[] = {{18000, 8, 32, 24, 512, 0}, {75000, 4, 32, 24, 512, 0}, {400000, 6, 64, 32, 512, 0},
+                               {kAnyCells, 4, 64, 22, 256, 0}};
+constexpr MtWindow kMtF16[] = {{18000, 8, 32, 24, 768, 0}, {60000, 4, 32, 24, 768, 0}, {300000, 6, 64, 32, 512, 0}};
+
+template <size_t n>
+const MtWindow* mt_pick(const MtWindow (&w)[n], uint64_t cells) {
+  for (const MtWindow& x : w)
+    if (cells <= x.cells) return &x;
+  return nullptr;
+}
+const MtWindow* mt_window(const flb_engine* h) {
+  const uint64_t cells = (uint64_t)h->N * h->peers;
+  if (h->s_size == 8) return mt_pick(kMtF64, cells);
+  if (h->s_size == 2) return mt_pick(kMtF16, cells);
+  return h->fused ? mt_pick(kMtF32, cells) : mt_pick(kMtF32Ref, cells);
+}
+
+// The launch of at most `left` steps (a.T of them) on windows w.
+MtArgs mt_plan(const flb_engine* h, const MtWindow& w, uint64_t left) {
+  MtArgs a{};
+  a.T = left < (uint64_t)w.T ? (int)left : w.T;
+  a.W = w.W;
+  a.H = w.H;
+  a.threads = w.threads;
+  a.pairs = w.pairs;
+  a.vec = h->nx % 4u == 0;  // rows move in groups of four cells
+  a.pad = a.vec ? (a.T + 3) / 4 * 4 : a.T;
+  a.OW = a.W - a.pad - a.T;
+  if (a.vec) a.OW = a.OW / 4 * 4;
+  a.OH = a.H - 2 * a.T;
+  a.bx = (int)((h->nx + (uint32_t)a.OW - 1) / (uint32_t)a.OW);
+  a.tiles = a.bx * (int)((h->ny + (uint32_t)a.OH - 1) / (uint32_t)a.OH);
+  return a;
+}
+
+// Whether this handle's steps can run several to a launch.
+bool mt_possible(const flb_engine* h) {
+  return !h->fs && !h->has_io && h->desc.kernel_variant == 0 && mt_window(h) != nullptr;
+}
+// ... and may now (not while the caller captures the stream: the launch
+// alternates between two buffers).
+bool mt_usable(flb_engine* h) {
+  if (!h->d_f2 || !mt_possible(h)) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(h->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+}
+
+// One launch of at most `left` steps, the last of which writes density and
+// velocity when it is the last of `left` (wm).
+flb_status mt_launch(flb_engine* h, uint64_t left, bool wm, int& T) {
+  MtArgs a = mt_plan(h, *mt_window(h), left);
+  refresh_params(h);
+  a.dst = h->d_f2;
+  a.t = (uint32_t)h->t;
+  a.wm = wm && (uint64_t)a.T == left;
+  cudaError_t e = cudaSuccess;
+  dispatch(h, [&](auto ops) { e = ops.mt(h, a); });
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return cuda_fail(h, e, "multi-step launch");
+  }
+  std::swap(h->d_f, h->d_f2);
+  T = a.T;
+  return FLB_OK;
+}
+
+constexpr int kMtGraph = 8;  // launches per graph (even: the buffers end where they began)
+
+flb_status mt_capture(flb_engine* h, GraphSlot& g, int T) {
+  FLB_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+  flb_status s = FLB_OK;
+  int t = 0;
+  for (int k = 0; k < kMtGraph && s == FLB_OK; k++) s = mt_launch(h, (uint64_t)T, false, t);
+  cudaGraph_t graph = nullptr;
+  cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
+  if (s == FLB_OK && e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
+  if (graph) cudaGraphDestroy(graph);
+  if (s != FLB_OK) return s;
+  if (e != cudaSuccess) return cuda_fail(h, e, "multi-step graph");
+  g.kernels = kMtGraph;
+  g.f = h->d_f;
+  return FLB_OK;
+}
+
+// n steps of the single phase; the last launch writes density and velocity.
+// Graphs of eight launches where many handles share the host thread that
+// launches them (48 cases on 16 streams: the launches took longer than the
+// kernels); a handle on its own is bound by the GPU, and FP16 storage needs
+// the step number in every launch.
+flb_status mt_steps(flb_engine* h, uint64_t n) {
+  const MtWindow& w = *mt_window(h);
+  const uint64_t per = (uint64_t)kMtGraph * (uint64_t)w.T;
+  while (n > 0) {
+    if (h->peers > 1 && h->s_size != 2 && n > per) {
+      GraphSlot& g = h->g_mt[2 * (h->d_f < h->d_f2 ? 0 : 1) + (int)(h->t & 1u)];
+      if (g.exec && g.f != h->d_f) destroy_graph(g);
+      if (!g.exec) {
+        const flb_status s = mt_capture(h, g, w.T);
+        if (s != FLB_OK) return s;
+      }
+      FLB_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
+      h->launches += g.kernels;
+      h->t += per;
+      n -= per;
+      continue;
+    }
+    int T = 0;
+    const flb_status s = mt_launch(h, n, true, T);
+    if (s != FLB_OK) return s;
+    h->launches += 1;
+    h->t += (uint64_t)T;
+    n -= (uint64_t)T;
+  }
+  refresh_params(h);
   return FLB_OK;
 }
 
@@ -410,9 +571,10 @@ flb_status check_persist(flb_engine* h) {
 }
 
 void free_all(flb_engine* h) {
+  for (GraphSlot& g : h->g_mt) destroy_graph(g);
   destroy_graph(h->g_pair);
   destroy_graph(h->g_big);
-  void* bufs[] = {h->d_f,          h->d_rho,         h->d_u,           h->d_flags[0],    h->d_flags[1],
+  void* bufs[] = {h->d_f,          h->d_f2,          h->d_rho,         h->d_u,           h->d_flags[0],    h->d_flags[1],
                   h->d_geo,        h->d_nbmask,      h->d_mass,        h->d_excess,      h->d_phi,
                   h->d_recon,      h->d_recon_mask,  h->d_rho_snap,    h->d_u_snap,      h->d_partial,
                   h->d_scalar,     h->d_counts,      h->d_nz,          h->d_lbits,       h->d_list[0][0],
@@ -559,6 +721,8 @@ void fill_case_constants(const flb_case_desc* desc, KParams& k) {
     volatile float hx = 0.5f * k.fx, hy = 0.5f * k.fy;
     k.fu_hfx = hx;
     k.fu_hfy = hy;
+    k.fu_nhfx = -hx;
+    k.fu_nhfy = -hy;
     k.fu_sw[0] = k.f16_scale * wgt<float>(0);  // exact: power-of-two scale
     k.fu_sw[1] = k.f16_scale * wgt<float>(1);
     k.fu_sw[2] = k.f16_scale * wgt<float>(5);
@@ -572,6 +736,12 @@ void fill_case_constants(const flb_case_desc* desc, KParams& k) {
 }
 
 flb_status validate_desc(const flb_case_desc* d, std::string& msg) { return validate(d, msg); }
+
+void set_peers(flb_engine* h, uint32_t peers) {
+  if (h->peers == peers) return;
+  for (GraphSlot& g : h->g_mt) destroy_graph(g);
+  h->peers = peers;
+}
 
 }  // namespace flb
 
@@ -745,6 +915,12 @@ FLB_API flb_status flb_create(const flb_case_desc* desc, flb_handle* out) {
     cudaError_t e = ++nalloc == fail_at ? cudaErrorMemoryAllocation : cudaMalloc(a.p, a.bytes);
     if (e != cudaSuccess) return bail(cuda_fail(h, e, "cudaMalloc"));
   }
+  // the second buffer of the multi-step kernel; without it (no memory) the
+  // handle runs one step per launch
+  if (mt_possible(h) && cudaMalloc(&h->d_f2, 9 * N * h->s_size) != cudaSuccess) {
+    cudaGetLastError();
+    h->d_f2 = nullptr;
+  }
   if (h->fs) {
     // list lengths start at zero
     cudaError_t e0 = cudaMemsetAsync(h->d_lcount, 0, 4 * sizeof(uint32_t), h->stream);
@@ -821,6 +997,10 @@ FLB_API flb_status flb_step(flb_handle h, uint64_t n) {
   nvtxRangePushA("flb_step");
   uint64_t remaining = n;
   flb_status s = FLB_OK;
+  if (n >= 2 && mt_usable(h)) {
+    s = mt_steps(h, n);
+    remaining = 0;
+  }
   while (remaining > 0 && s == FLB_OK) {
     // graphs cover pairs of steps from an even t; the last step of the call
     // runs on its own so that it writes density and velocity

@@ -24,12 +24,18 @@ namespace flb {
 // engine.cu: descriptor checks and per-case constants shared with the batch
 flb_status validate_desc(const flb_case_desc* d, std::string& msg);
 void fill_case_constants(const flb_case_desc* desc, KParams& k);
+// how many handles are stepped concurrently with this one, itself included
+// (its stream idle)
+void set_peers(flb_engine* h, uint32_t peers);
 
 // stream-collide; vec selects the V-cells-per-thread data path, fu the fused
 // SRT arithmetic
 template <class S, class C, class M>
 void launch_sc(const KParams& kp, cudaStream_t st, uint32_t odd, bool fs, bool hw, bool wm, bool vec, bool fu);
 int vec_width(int precision);
+// single phase: a.T steps in one launch
+template <class S, class C, class M>
+cudaError_t launch_mt(const KParams& kp, const MtArgs& a, cudaStream_t st, bool fu);
 // free surface: the listed super-tiles in a persistent grid of `grid` blocks;
 // vec: the vector data path (needs nx divisible by the vector width)
 template <class S, class C, class M>

@@ -1,0 +1,68 @@
+"""The single-phase multi-step kernel (several time steps per launch) against
+the CPU oracle: every value of the population array, density and velocity equal."""
+import numpy as np
+import pytest
+
+from flowlb_b200 import cases
+from flowlb_b200 import engine as E
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def pair(flags, variant, bb, arith, **kw):
+    prec = {O.F64: 64, O.F32: 32, O.F16S: 16}[variant]
+    s = E.Solver(flags, precision=prec, bounce_back=bb, arithmetic=arith, **kw)
+    o = O.Oracle(flags, O.OracleConfig(variant=variant, bb=bb, arithmetic=arith, **kw))
+    return s, o
+
+
+def check(s, o, variant, what):
+    f = o.f64() if variant == O.F64 else o.f64().astype(np.float32)
+    for name, a, b in (("f", s.f, f), ("rho", s.rho, o.rho), ("u", s.u, o.u)):
+        assert np.array_equal(a, b), f"{what}: {name} differs at {np.flatnonzero(a != b)[:5]}"
+
+
+# widths and heights below, at and beyond a window, whole vectors and not; one
+# grid per window size the dispatch picks
+@pytest.mark.parametrize("nx,ny", [(3, 5), (17, 9), (64, 40), (101, 61), (256, 64), (517, 131), (1024, 136)],
+                         ids=lambda v: str(v))
+@pytest.mark.parametrize("variant", [O.F32, O.F64, O.F16S], ids=["f32", "f64", "f16s"])
+@pytest.mark.parametrize("bb,arith", [(E.BB_HALFWAY, E.ARITH_FUSED), (E.BB_IMPLICIT, E.ARITH_REFERENCE)],
+                         ids=["halfway-fused", "implicit-ref"])
+def test_multi_step_matches_oracle(nx, ny, variant, bb, arith):
+    w = max(1, nx // 5)
+    flags = cases.channel_with_block(nx, ny, nx // 3, nx // 3 + w, max(2, ny // 3))
+    flags[ny // 2, nx // 2] = cases.GAS  # not updated, not a wall
+    s, o = pair(flags, variant, bb, arith, tau=0.58, fx=2e-5, fy=-1e-5)
+    for n in (1, 2, 21, 8, 3):  # odd and even starts, whole launches and remainders
+        s.step(n)
+        o.step(n)
+        check(s, o, variant, f"t={o.t}")
+    s.close()
+
+
+@pytest.mark.parametrize("kw", [dict(u_max=0.01), dict(subgrid=True), dict(collision=1, use_force=False)],
+                         ids=["limiter", "subgrid", "trt"])
+def test_multi_step_options_match_oracle(kw):
+    c = cases.plain_channel(200, 48)
+    s, o = pair(c.flags, O.F32, E.BB_HALFWAY, E.ARITH_FUSED, tau=0.55, fx=1e-4, **kw)
+    s.step(67)
+    o.step(67)
+    check(s, o, O.F32, str(kw))
+    s.close()
+
+
+def test_multi_step_large_grid_equals_one_step_per_launch():
+    """A grid on the large-grid window (several windows wide and high), against the one-step kernels."""
+    c = cases.plain_channel(2052, 600)
+    for prec in (32, 64, 16):
+        a = E.Solver(c.flags, precision=prec, tau=0.6, fx=1e-5)
+        b = E.Solver(c.flags, precision=prec, tau=0.6, fx=1e-5, kernel_variant=1)
+        for n in (37, 6):
+            a.step(n)
+            b.step(n)
+        for fid in (E.FIELD_F, E.FIELD_RHO, E.FIELD_U):
+            assert np.array_equal(a.read(fid), b.read(fid)), (prec, fid)
+        a.close()
+        b.close()
