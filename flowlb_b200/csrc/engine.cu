@@ -44,7 +44,8 @@ struct GraphSlot {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   uint64_t kernels = 0;
-  const void* f = nullptr;  // population buffer it was captured with
+  const void* f = nullptr;    // population and density buffers it was captured with
+  const void* rho = nullptr;
 };
 
 }  // namespace
@@ -114,6 +115,7 @@ struct flb_engine {
   uint8_t* d_recon_mask = nullptr;
   void* d_rho_snap = nullptr;
   void* d_u_snap = nullptr;
+  bool snap_same = false;  // single phase: the never-written cells hold the same in d_rho, d_u and their snapshots
   double* d_partial = nullptr;
   double* d_scalar = nullptr;
   unsigned long long* d_counts = nullptr;
@@ -282,15 +284,33 @@ ListClear list_clear(flb_engine* h, uint64_t t) {
   return ListClear{nl.counts, nl.bits, h->nwords};
 }
 
+// The density and velocity of the last step into the snapshot that inlet and
+// outlet cells read.
+void copy_snap(flb_engine* h) {
+  cudaMemcpyAsync(h->d_rho_snap, h->d_rho, (size_t)h->N * h->c_size, cudaMemcpyDeviceToDevice, h->stream);
+  cudaMemcpyAsync(h->d_u_snap, h->d_u, 2ull * h->N * h->c_size, cudaMemcpyDeviceToDevice, h->stream);
+  h->snap_same = true;
+}
+
 // Issues the passes of one time step at t on the stream.
 uint64_t issue_step(flb_engine* h, uint64_t t, bool write_macro) {
   const uint32_t odd = (uint32_t)(t & 1u);
   uint64_t k = 0;
-  refresh_params(h);
   if (h->has_io) {
-    cudaMemcpyAsync(h->d_rho_snap, h->d_rho, (size_t)h->N * h->c_size, cudaMemcpyDeviceToDevice, h->stream);
-    cudaMemcpyAsync(h->d_u_snap, h->d_u, 2ull * h->N * h->c_size, cudaMemcpyDeviceToDevice, h->stream);
+    // inlet and outlet cells read the last step's density and velocity of
+    // their neighbours, which this step rewrites.  Single phase: every step
+    // writes those of every updated cell, so two pairs of buffers alternate (the
+    // cells that are never written hold the same in both; 4001x41 F32 in the
+    // reference's modes, 200 steps and the read-back on a B200: 8.8 us per step
+    // copying both arrays before every step, 5.3 alternating).  Free surface: which cells are written changes,
+    // so the arrays are copied.
+    if (h->fs || !h->snap_same) copy_snap(h);
+    if (!h->fs) {
+      std::swap(h->d_rho, h->d_rho_snap);
+      std::swap(h->d_u, h->d_u_snap);
+    }
   }
+  refresh_params(h);
   if (h->fs) {
     h->kp.trust_prev = h->trust ? 1 : 0;
     const FsLists L = fs_lists(h, t);
@@ -366,7 +386,7 @@ void destroy_graph(GraphSlot& g) {
 // Captures 2*pairs steps starting at an even t with flag buffer 0 current:
 // the passes of every step, or one persistent launch (free surface, h->persist).
 flb_status capture(flb_engine* h, GraphSlot& g, int pairs) {
-  if (g.exec && g.f == h->d_f) return FLB_OK;
+  if (g.exec && g.f == h->d_f && g.rho == h->d_rho) return FLB_OK;
   destroy_graph(g);
   const int saved_cur = h->cur;
   FLB_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
@@ -399,6 +419,7 @@ flb_status capture(flb_engine* h, GraphSlot& g, int pairs) {
   g.exec = exec;
   g.kernels = kernels;
   g.f = h->d_f;
+  g.rho = h->d_rho;
   return FLB_OK;
 }
 
@@ -636,6 +657,7 @@ flb_status initialise(flb_engine* h) {
   FLB_CUDA(h, cudaMemsetAsync(h->d_f, 0, 9ull * h->N * h->s_size, h->stream));
   h->cur = 0;
   h->t = 0;
+  h->snap_same = false;
   if (h->fs)
     launch_init_flags(h->d_geo, h->d_flags[0], h->nx, h->ny, 1, h->d_mass, h->d_excess, h->d_phi, h->m_size == 8,
                       h->stream);
@@ -995,6 +1017,7 @@ FLB_API flb_status flb_step(flb_handle h, uint64_t n) {
     }
   }
   nvtxRangePushA("flb_step");
+  if (h->has_io && !h->fs && !h->snap_same) copy_snap(h);  // (here: not into a graph of steps)
   uint64_t remaining = n;
   flb_status s = FLB_OK;
   if (n >= 2 && mt_usable(h)) {
@@ -1198,6 +1221,7 @@ FLB_API flb_status flb_write_field(flb_handle h, int field, const void* src, int
     FLB_CUDA(h, cudaMemcpyAsync(dst, src, bytes, kind, h->stream));
   }
   if (field == FLB_FIELD_FLAGS) refresh_plain(h);
+  h->snap_same = false;
   h->trust = false;
   h->lists_valid = false;
   FLB_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -1549,6 +1573,7 @@ FLB_API flb_status flb_load_checkpoint(flb_handle h, const char* path) {
   std::fclose(fp);
   h->t = hd.t;
   h->cur = cur;
+  h->snap_same = false;
   h->trust = false;
   h->lists_valid = false;
   refresh_params(h);
