@@ -20,6 +20,7 @@
 #include <type_traits>
 
 #include "launch.h"
+#include "pair.cuh"
 #include "sc_cell.cuh"
 
 // occupancy targets (resident blocks per SM) of the two data paths
@@ -484,23 +485,28 @@ __device__ __forceinline__ void h16_cells(const KParams& p, const uint32_t x0, c
         }
       }
     }
-    const DevOut oa = collide_fused_dev<LIM>(ha, invS, p.inv_tau, p.fu_omc, p.fu_nk3, p.fu_hfx, p.fu_hfy, p.fu_fx,
-                                             p.fu_fy, p.u_max, p.fu_g, p.fu_h, p.fu_sw);
-    const DevOut ob = collide_fused_dev<LIM>(hb, invS, p.inv_tau, p.fu_omc, p.fu_nk3, p.fu_hfx, p.fu_hfy, p.fu_fx,
-                                             p.fu_fy, p.u_max, p.fu_g, p.fu_h, p.fu_sw);
+    f2 h[9];
+#pragma unroll
+    for (int i = 0; i < 9; i++) h[i] = pack(ha[i], hb[i]);
+    const PairMacro o = collide_fused_dev_pair<LIM>(h, p);
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+      ha[i] = lo(h[i]);
+      hb[i] = hi(h[i]);
+    }
     const uint32_t idx = row + x0 + 2 * P;
     if (WM) {
       float* R = static_cast<float*>(p.rho);
       float* U = static_cast<float*>(p.u);
       if (upd[P] & 1u) {
-        R[idx] = oa.rho;
-        U[idx] = oa.ux;
-        U[idx + p.N] = oa.uy;
+        R[idx] = lo(o.rho);
+        U[idx] = lo(o.ux);
+        U[idx + p.N] = lo(o.uy);
       }
       if (upd[P] >> 16) {
-        R[idx + 1] = ob.rho;
-        U[idx + 1] = ob.ux;
-        U[idx + 1 + p.N] = ob.uy;
+        R[idx + 1] = hi(o.rho);
+        U[idx + 1] = hi(o.ux);
+        U[idx + 1 + p.N] = hi(o.uy);
       }
     }
     // stochastic rounding of the pair (idx is even: row and x0 are)

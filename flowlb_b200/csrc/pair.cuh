@@ -112,4 +112,48 @@ __device__ __forceinline__ PairMacro collide_fused_pair(f2* f, const KParams& p)
   return m;
 }
 
+// collide_fused_dev (lattice.cuh), operation by operation.
+template <bool LIM>
+__device__ __forceinline__ PairMacro collide_fused_dev_pair(f2* h, const KParams& p) {
+  const f2 s12 = h[1] + h[2], s34 = h[3] + h[4], s56 = h[5] + h[6], s78 = h[7] + h[8];
+  const f2 d12 = h[2] - h[1], d34 = h[4] - h[3], d56 = h[6] - h[5], d78 = h[8] - h[7];
+  const f2 dS = ((h[0] + s12) + (s34 + s56)) + s78;
+  const f2 jx = (d12 + d56) + d78, jy = (d34 + d56) - d78;
+  const f2 invS = both(p.f16_inv);
+  const f2 delta = dS * invS;
+  PairMacro m;
+  m.rho = fmac(dS, invS, both(1.0f));
+  const f2 inv = neg_rcp(m.rho);
+  const f2 invs = inv * invS;
+  f2 ux = fmac(both(p.fu_nhfx), inv, jx * invs), uy = fmac(both(p.fu_nhfy), inv, jy * invs);
+  if (LIM) {
+    float ax = lo(ux), ay = lo(uy), bx = hi(ux), by = hi(uy);
+    limit_u(p.u_max, ax, ay);
+    limit_u(p.u_max, bx, by);
+    ux = pack(ax, bx);
+    uy = pack(ay, by);
+  }
+  m.ux = ux;
+  m.uy = uy;
+  const f2 usq = fmac(ux, ux, uy * uy);
+  const f2 uF = fmac(ux, both(p.fu_fx), uy * both(p.fu_fy));
+  const f2 A = both(p.inv_tau) * m.rho;
+  const f2 t1 = fmac(both(-1.5f), usq, both(1.0f));
+  const f2 x = fmac(delta, t1, both(-1.5f) * usq);
+  const f2 Bd = fmac(both(p.inv_tau), x, both(p.fu_nk3) * uF);
+  const f2 A3 = both(3.0f) * A, A45 = both(4.5f) * A;
+  h[0] = fmac(both(p.fu_omc), h[0], both(p.fu_sw[0]) * Bd);
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int i = 2 * q + 1;
+    const f2 cu = q == 0 ? ux : (q == 1 ? uy : (q == 2 ? ux + uy : ux - uy));
+    const f2 E = fmac(cu, fmac(A45, cu, both(p.fu_h[q])), Bd);
+    const f2 O = fmac(A3, cu, both(p.fu_g[q]));
+    const f2 swi = both(p.fu_sw[q < 2 ? 1 : 2]);
+    h[i] = fmac(both(p.fu_omc), h[i], swi * (E + O));
+    h[i + 1] = fmac(both(p.fu_omc), h[i + 1], swi * (E - O));
+  }
+  return m;
+}
+
 }  // namespace flb
