@@ -38,12 +38,14 @@
 namespace flb {
 namespace {
 
-constexpr int kAdjBlock = 256;
-// resident blocks per SM the reverse step is compiled for: four (at most 64
-// registers a thread; the FP64 step spills 44 bytes) measured faster than the
-// 92-register build's two on a B200 (FP64 backward of the 1024x256 case 68.1
-// -> 62.7 ms; three blocks, 80 registers: 67.4 ms)
-constexpr int kAdjBwdBlocks = 4;
+constexpr int kAdjBlock = 128;
+// resident blocks per SM the steps are compiled for.  Measured on a B200
+// (128-thread blocks, us per step): the reverse step at eight (64 registers;
+// FP64 spills) 14.0 on the 1024x256 FP64 case, 14.5 at five (100 registers, no
+// spills; 256-thread blocks at four: 14.3); on a grid whose blocks are all
+// resident at five per SM, five: 517x131 FP64 4.9 against 6.3.  FP32 fits 64
+// registers either way.  Forward: 5.0 at eight (256-thread blocks: 5.3).
+constexpr int kAdjFwdBlocks = 8, kAdjBwdBlocks = 8, kAdjBwdFew = 5;
 // opposite direction (directions of lattice.cuh: i and i+1 opposite for odd i)
 __host__ __device__ constexpr int opp(int i) { return i == 0 ? 0 : ((i & 1) ? i + 1 : i - 1); }
 
@@ -138,27 +140,35 @@ __device__ __forceinline__ Cell<T> cell_state(const AdjParams<T>& p, const T* f,
 }
 
 
-// One forward step fin -> fout.  obj: add rho u_x of the last column to jrow.
+// One forward step fin -> fout (fin null: the segment's checkpoint).  jrow: rho
+// u_x of the last column is added to it.
 // ckpt (segment's first step only): the input state is also copied there.
 template <class T>
-__global__ void __launch_bounds__(kAdjBlock) k_por_fwd(const AdjParams<T> p, const T* __restrict__ fin,
+__global__ void __launch_bounds__(kAdjBlock, kAdjFwdBlocks) k_por_fwd(const __grid_constant__ AdjParams<T> p, const T* fin,
                                                        T* __restrict__ fout, double* __restrict__ jrow,
                                                        const SegDesc* __restrict__ seg, uint32_t j, int copy_ckpt,
                                                        T* __restrict__ mac) {
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-  if (x >= p.nx) return;
-  const uint32_t idx = x + y * p.nx, N = p.N;
+  const bool in = x < p.nx;
+  const uint32_t idx = in ? x + y * p.nx : 0u, N = p.N;
+  // what the step before does not write is loaded before waiting for it
+  const uint8_t flag = p.flags[idx];
+  const uint32_t sw = p.srcw[idx];
+  const T s = p.s[idx], id = p.id[idx];
+  pdl_wait();
+  pdl_trigger();
+  if (!in) return;
+  if (!fin) fin = static_cast<const T*>(seg->ckpt);
   if (copy_ckpt) {
     T* ck = static_cast<T*>(seg->ckpt);
 #pragma unroll
     for (int i = 0; i < 9; i++) ck[(uint32_t)i * N + idx] = fin[(uint32_t)i * N + idx];
   }
-  if (p.flags[idx] & kWall) return;
+  if (flag & kWall) return;
   const Nb nb = sources(x, y, p.nx, p.ny);
   T f[9];
-  gather(p, fin, idx, p.srcw[idx], nb, f);
-  const T s = p.s[idx];
-  const Cell<T> c = cell_state(p, f, s, p.id[idx]);
+  gather(p, fin, idx, sw, nb, f);
+  const Cell<T> c = cell_state(p, f, s, id);
   if (mac) {  // the backward step's inputs: rho and v = j / rho
     mac[idx] = c.rho;
     mac[N + idx] = c.vx;
@@ -186,30 +196,41 @@ __global__ void __launch_bounds__(kAdjBlock) k_por_fwd(const AdjParams<T> p, con
   }
 }
 
+// The steps of a segment are launched so that a step's blocks may be scheduled
+// while the one before drains (launch_pdl); each waits for it before its first
+// read of what it wrote.  Measured on a B200 against ordinary launches, us per
+// step forward / backward: 160x60 F32 2.3/3.4 -> 1.65/2.9, 517x131 F32 3.0/5.7
+// -> 2.4/4.6, 1024x256 FP64 6.0/15.8 -> 5.0/14.0 (with the 128-thread blocks).
+
 // One backward step: mac holds rho, v_x, v_y of step t (written by its forward
 // recomputation), lam_next = dJ/d(output of step t), lam = dJ/d(input of step
 // t) (scattered).  sbar: dJ/ds per cell; gpart: dJ/dg per block (2 doubles per
 // block).  The update's derivative needs no population itself, only rho and v.
-template <class T>
-__global__ void __launch_bounds__(kAdjBlock, kAdjBwdBlocks) k_por_bwd(const AdjParams<T> p, const T* __restrict__ mac,
+template <class T, int MB>
+__global__ void __launch_bounds__(kAdjBlock, MB) k_por_bwd(const __grid_constant__ AdjParams<T> p, const T* __restrict__ mac,
                                                        const T* __restrict__ lam_next, T* __restrict__ lam,
                                                        double* __restrict__ sbar, double* __restrict__ gpart,
                                                        const SegDesc* __restrict__ seg, uint32_t j) {
   __shared__ double red[2][kAdjBlock / 32];
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   double gxb_d = 0.0, gyb_d = 0.0;
-  if (x < p.nx) {
-    const uint32_t idx = x + y * p.nx, N = p.N;
-    if (!(p.flags[idx] & kWall)) {
-      const uint32_t sw = p.srcw[idx];
+  const bool in = x < p.nx;
+  const uint32_t idx = in ? x + y * p.nx : 0u, N = p.N;
+  // what the step before does not write is loaded before waiting for it
+  const uint8_t flag = p.flags[idx];
+  const uint32_t sw = p.srcw[idx];
+  const T s = p.s[idx], id = p.id[idx];
+  Cell<T> c;
+  c.rho = mac[idx];
+  c.vx = mac[N + idx];
+  c.vy = mac[2 * N + idx];
+  pdl_wait();
+  pdl_trigger();
+  if (in) {
+    if (!(flag & kWall)) {
       const Nb nb = sources(x, y, p.nx, p.ny);
-      const T s = p.s[idx];
-      Cell<T> c;
-      c.rho = mac[idx];
       c.ir = T(1) / c.rho;
-      c.vx = mac[N + idx];
-      c.vy = mac[2 * N + idx];
-      cell_rest(p, c, s, p.id[idx]);
+      cell_rest(p, c, s, id);
       const T base = T(1) - T(1.5) * c.usq;
       T fb[9];
       const T m0 = lam_next[idx];
@@ -331,13 +352,6 @@ template <class T>
 __global__ void k_por_fill(T* f, uint32_t N, int zero) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < 9 * N) f[k] = zero ? T(0) : wq<T>((int)(k / N));
-}
-
-// tape[0] = checkpoint of the segment
-template <class T>
-__global__ void k_por_load(T* dst, const SegDesc* __restrict__ seg, uint32_t n) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) dst[k] = static_cast<const T*>(seg->ckpt)[k];
 }
 
 __global__ void k_srcw(const uint8_t* __restrict__ flags, uint8_t* __restrict__ srcw, uint32_t nx, uint32_t ny) {
@@ -480,22 +494,25 @@ flb_status capture(flb_adjoint a) {
   adrop_graphs(a);
   const AdjParams<T> p = params<T>(a);
   const dim3 grid(a->gx_blocks, a->ny), block(kAdjBlock);
-  const uint32_t N = a->N, K = a->K, n9 = 9 * N, n3 = 3 * N;
+  const uint32_t N = a->N, K = a->K, n3 = 3 * N;
   T* st[2] = {static_cast<T*>(a->d_state[0]), static_cast<T*>(a->d_state[1])};
   T* rs[2] = {static_cast<T*>(a->d_rstate[0]), static_cast<T*>(a->d_rstate[1])};
   T* lam[2] = {static_cast<T*>(a->d_lam[0]), static_cast<T*>(a->d_lam[1])};
   T* tape[2] = {static_cast<T*>(a->d_tape), static_cast<T*>(a->d_tape) + (size_t)K * n3};
   auto emit_rec = [&](cudaStream_t sm, int b) {
-    k_por_load<T><<<(n9 + 255) / 256, 256, 0, sm>>>(rs[0], a->d_seg + 1, n9);
     for (uint32_t j = 0; j < K; j++)
-      k_por_fwd<T><<<grid, block, 0, sm>>>(p, rs[j & 1], rs[(j + 1) & 1], nullptr, a->d_seg + 1, j, 0,
-                                          tape[b] + (size_t)j * n3);
+      launch_pdl(k_por_fwd<T>, grid, block, sm, p, (const T*)(j == 0 ? nullptr : rs[j & 1]), rs[(j + 1) & 1],
+                 (double*)nullptr, (const SegDesc*)(a->d_seg + 1), j, 0, tape[b] + (size_t)j * n3);
   };
+  int nsm = 1;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, a->device);
+  const bool few = sizeof(T) == 8 && a->nblocks <= (uint32_t)(nsm * kAdjBwdFew);
+  auto* bwd = few ? k_por_bwd<T, kAdjBwdFew> : k_por_bwd<T, kAdjBwdBlocks>;
   auto emit_back = [&](cudaStream_t sm, int b) {
     for (uint32_t q = 0; q < K; q++) {
       const uint32_t j = K - 1 - q;
-      k_por_bwd<T><<<grid, block, 0, sm>>>(p, tape[b] + (size_t)j * n3, lam[q & 1], lam[(q + 1) & 1], a->d_sbar,
-                                          a->d_gpart, a->d_seg, j);
+      launch_pdl(bwd, grid, block, sm, p, (const T*)(tape[b] + (size_t)j * n3), (const T*)lam[q & 1],
+                 lam[(q + 1) & 1], a->d_sbar, a->d_gpart, (const SegDesc*)a->d_seg, j);
     }
   };
   auto finish = [&](cudaGraphExec_t* out) -> flb_status {
@@ -509,8 +526,8 @@ flb_status capture(flb_adjoint a) {
   flb_status s;
   FLB_ACUDA(a, cudaStreamBeginCapture(a->stream, cudaStreamCaptureModeThreadLocal));
   for (uint32_t j = 0; j < K; j++)
-    k_por_fwd<T><<<grid, block, 0, a->stream>>>(p, st[j & 1], st[(j + 1) & 1], a->d_jrow, a->d_seg, j, j == 0,
-                                                nullptr);
+    launch_pdl(k_por_fwd<T>, grid, block, a->stream, p, (const T*)st[j & 1], st[(j + 1) & 1], a->d_jrow,
+               (const SegDesc*)a->d_seg, j, (int)(j == 0), (T*)nullptr);
   if ((s = finish(&a->g_fwd)) != FLB_OK) return s;
   for (int b = 0; b < 2; b++) {
     FLB_ACUDA(a, cudaStreamBeginCapture(a->stream, cudaStreamCaptureModeThreadLocal));
