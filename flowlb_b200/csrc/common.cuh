@@ -88,14 +88,11 @@ __device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_
 // visit (NextLists), and the next step's passes loop over the lists in a
 // persistent grid.  all = 1 visits every super-tile (first step after the
 // state was set from outside).
-constexpr uint32_t kSTW = 128, kSTH = 8;
-// threads per block of the listed stream-collide and FS_1 kernels: 1024 take
-// a super-tile in one pass (one cell per thread), 256 in four (row chunks)
-#ifndef FLB_LIST_BLOCK
-#define FLB_LIST_BLOCK 1024
-#endif
-constexpr int kListBlock = FLB_LIST_BLOCK;
-
+// 64 x 8 cells: with 128 x 8 the about 320 super-tiles of a 2048x512 dam break
+// were one round and a bit of blocks, and small grids ran on a few SMs
+// (measured with the forms of k_fs.cu and k_sc.cu, us per step, 128 -> 64 wide:
+// 101x101 17.8 -> 13.8, 2048x512 26.7 -> 23.4, 8192x2048 239 -> 232).
+constexpr uint32_t kSTW = 64, kSTH = 8;
 struct TileList {
   const uint32_t* list;
   const uint32_t* count;
@@ -244,6 +241,20 @@ __device__ __forceinline__ void prefetch_super_tile(const KParams& p, uint32_t t
   }
   if (row < 0 || row >= (int)p.ny) return;
   l2_prefetch_inward(base + ((size_t)row * p.nx + x0) * elem, w * elem);
+}
+
+// The parameters of an odd step for a kernel compiled for even ones: the two
+// slots of every direction pair trade places.  The free-surface kernels are
+// compiled for one parity only: a step runs each pass's long, mostly
+// straight-line code once per block, and the passes of both parities together
+// did not stay in the SMs' instruction caches from step to step (on a tile of
+// its own the flag stencil took 5,000 cycles, nearly all of it waiting for
+// instructions).
+inline KParams as_even(const KParams& kp, uint32_t odd) {
+  KParams q = kp;
+  if (odd)
+    for (int i = 1; i < 9; i += 2) std::swap(q.slot[i], q.slot[i + 1]);
+  return q;
 }
 
 template <class S>

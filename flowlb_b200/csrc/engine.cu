@@ -31,13 +31,17 @@ enum Variant { V_F64 = 0, V_F32 = 1, V_F16S = 2, V_F32M32 = 3 };
 
 constexpr int kGraphPairs = 16;  // steps per large graph = 2 * kGraphPairs
 // FLB_STEP_AUTO runs the free-surface step as one persistent kernel on grids of
-// up to this many super-tiles.  Measured on a B200 (2048x512 dam break, 1024
-// super-tiles): 34.8 us per step persistent against 29.3 us for the PDL-chained
-// per-pass kernels.  FS_1 needs 64 registers, so the persistent kernel keeps
-// 1024 threads per SM where the per-pass stream-collide and flag kernels keep
-// 2048, and each of its four grid barriers per step costs about 1.5 us; AUTO
-// therefore runs the per-pass kernels everywhere (0 super-tiles).
+// up to this many super-tiles.  Measured on a B200 (2048x512 dam break): 31 us
+// per step persistent against 23.4 us for the PDL-chained per-pass kernels;
+// 64x48, one super-tile per CTA: 16.0 against 13.  The persistent kernel keeps
+// 1024 threads per SM in every pass, and each of its three grid barriers per
+// step costs about 1.5 us; AUTO therefore runs the per-pass kernels everywhere
+// (0 super-tiles).  (As one thread-block cluster of 16 CTAs with the hardware
+// barrier, small grids only: 64x48 13.6, 101x101 17.3 against 14.3.)
 constexpr uint32_t kPersistAutoTiles = 0;
+// Up to this many super-tiles FS_1 and the flag pass take one cell per thread
+// (k_fs.cu).
+constexpr uint32_t kSmallTiles = 1024;
 constexpr uint32_t kPersistWaitLimit = 1u << 22;  // barrier polls before the persistent step gives up
 
 struct GraphSlot {
@@ -61,7 +65,8 @@ struct flb_engine {
   bool fs = false, hw = false, has_io = false;
   bool use_vec = false;       // vectorised stream-collide (single phase)
   bool use_vec_list = false;  // vectorised listed stream-collide (free surface)
-  int fs_form = FS_FORM_W128X1;  // launch form of the flag pass (FsForm)
+  bool fs_one_cell = false;          // FS_1 with one cell per thread
+  int fs_form = FS_FORM_W64X2;  // launch form of the flag pass (FsForm)
   bool fused = false;    // fused SRT arithmetic in stream-collide
   uint64_t t = 0;
   uint64_t launches = 0;
@@ -171,15 +176,17 @@ struct Ops {
     launch_sc_list<S, C, M>(h->kp, h->stream, odd, h->hw, tl, h->grid_sc, h->fused, h->use_vec_list);
   }
   static void fs1(flb_engine* h, uint32_t odd, const TileList& tl, const ListClear& lc) {
-    launch_fs1<S, C, M>(h->kp, h->stream, odd, h->hw, tl, h->grid_fs1, lc);
+    launch_fs1<S, C, M>(h->kp, h->stream, odd, h->hw, tl, h->grid_fs1, lc, h->fs_one_cell);
   }
   static int fs234(flb_engine* h, uint32_t odd, const TileList& tl, const NextLists& nl) {
     return launch_fs234<S, C, M>(h->kp, h->stream, odd, tl, h->grid_fs234, h->d_nz, nl, h->fs_form);
   }
+  // one round of resident blocks, no more than there are super-tiles (blocks
+  // without one cost their launch: 64x48 18.2 -> 16.4 us per step)
   static void grids(flb_engine* h, int nsm) {
-    h->grid_sc = (uint32_t)(nsm * sc_list_blocks_per_sm<S, C, M>(h->use_vec_list));
-    h->grid_fs1 = (uint32_t)(nsm * fs_blocks_per_sm<S, C, M>(0, 0));
-    h->grid_fs234 = (uint32_t)(nsm * fs_blocks_per_sm<S, C, M>(1, h->fs_form));
+    h->grid_sc = std::min(h->ntiles, (uint32_t)(nsm * sc_list_blocks_per_sm<S, C, M>(h->use_vec_list, h->ntiles)));
+    h->grid_fs1 = std::min(h->ntiles, (uint32_t)(nsm * fs_blocks_per_sm<S, C, M>(0, h->fs_one_cell ? 1 : 2)));
+    h->grid_fs234 = std::min(h->ntiles, (uint32_t)(nsm * fs_blocks_per_sm<S, C, M>(1, h->fs_form)));
   }
   static cudaError_t mt(flb_engine* h, const MtArgs& a) {
     if constexpr (std::is_same<S, float>::value && std::is_same<M, float>::value)
@@ -842,29 +849,16 @@ FLB_API flb_status flb_create(const flb_case_desc* desc, flb_handle* out) {
     const uint64_t tiles = (uint64_t)((desc->nx + kSTW - 1) / kSTW) * ((desc->ny + kSTH - 1) / kSTH);
     h->use_vec_list = desc->kernel_variant == 2 ||
                       (desc->kernel_variant == 0 && desc->nx % V == 0 && desc->precision == 16 && fused &&
-                       tiles > 4096u);
-    // flag pass: 128-wide tiles with two cells per thread (512-thread
-    // blocks, two per SM) on grids of up to 4096 super-tiles, 64-wide tiles
-    // with two cells per thread (256-thread blocks, five per SM at 48
-    // registers) above.  Measured on a B200 (quiet tiles counting their
-    // neighbours from the flags): 2048x512 dam break 25.9 us per step with
-    // 128x2 against 28.0 with 128x1, 28.0 with 64x1, 33.4 with 64x2 and 33.5
-    // with 128x4; 8192x2048 224.5 with 64x2 against 226.9 with 128x2, 232.1
-    // with 64x1 and 242.0 with 128x1.  Earlier builds (before the quiet-tile
-    // path): 2048x512 one cell per thread 29.2, two 30.1, four 34.6;
-    // 8192x2048 flag pass 110 us per step with two cells per thread at two
-    // blocks per SM (114 at three, 119 at four), one cell per thread 124,
-    // four 131, 32-wide tiles 158.  FLB_FS_FLAG_FORM (32, 64x1, 64x2, 128x1,
-    // 128x2 or 128x4: tile width x cells per thread) selects another form,
-    // with the same results.
-    h->fs_form = tiles <= 4096u ? FS_FORM_W128X2 : FS_FORM_W64X2;
+                       tiles > 8192u);
+    // FS_1 and the flag pass: one cell per thread on grids of up to
+    // kSmallTiles super-tiles, two above (FsForm, k_fs.cu).
+    // FLB_FS_FLAG_FORM selects another flag-pass form, with the same results.
+    h->fs_one_cell = tiles <= kSmallTiles;
+    h->fs_form = h->fs_one_cell ? FS_FORM_W64X1 : FS_FORM_W64X2;
     if (const char* v = std::getenv("FLB_FS_FLAG_FORM")) {
       if (!std::strcmp(v, "32")) h->fs_form = FS_FORM_W32;
-      else if (!std::strcmp(v, "128x1")) h->fs_form = FS_FORM_W128X1;
-      else if (!std::strcmp(v, "128x2")) h->fs_form = FS_FORM_W128X2;
-      else if (!std::strcmp(v, "128x4")) h->fs_form = FS_FORM_W128X4;
-      else if (!std::strcmp(v, "64x1")) h->fs_form = FS_FORM_W64X1;
-      else if (!std::strcmp(v, "64x2")) h->fs_form = FS_FORM_W64X2;
+      else if (!std::strcmp(v, "64x1") || !std::strcmp(v, "128x1")) h->fs_form = FS_FORM_W64X1;
+      else if (!std::strcmp(v, "64x2") || !std::strcmp(v, "128x2") || !std::strcmp(v, "128x4")) h->fs_form = FS_FORM_W64X2;
     }
   }
   s = check_io(h, desc->flags);

@@ -133,30 +133,22 @@ __device__ __forceinline__ void fs1_cell(const KParams& p, uint32_t x, uint32_t 
 // of kTX x 8 cells stages the flags of its 3-cell halo in shared memory and
 // evaluates the chain there, so neighbour flags are never read while another
 // block rewrites them.  Reads p.flags, writes p.flags_out.
-// Tiles of the flag pass: 128 x 8 (a whole super-tile) or 32 x 8 (a quarter,
-// the super-tile's four quarters in turn), with one, two or four cells per
-// thread (FsForm; the host picks by the grid's super-tile count).  On grids
-// of up to kWideTiles super-tiles the pass is launched with programmatic
-// dependent launch.
+// Tiles of the flag pass: 64 x 8 (a super-tile) with one or two cells per
+// thread, or 32 x 8 (its halves in turn) with one (FsForm; the host picks by
+// the grid's super-tile count).  On grids of up to kWideTiles super-tiles the
+// pass is launched with programmatic dependent launch.
 constexpr int kTY = 8, kHalo = 3;
 #ifndef FLB_FS_PDL_TILES
-#define FLB_FS_PDL_TILES 4096
+#define FLB_FS_PDL_TILES 8192
 #endif
 constexpr uint32_t kWideTiles = FLB_FS_PDL_TILES;
-#ifndef FLB_FS_WIDE_MIN_BLOCKS
-#define FLB_FS_WIDE_MIN_BLOCKS 2
-#endif
-#ifndef FLB_FS_HALF_MIN_BLOCKS
-#define FLB_FS_HALF_MIN_BLOCKS 2
-#endif
 #ifndef FLB_FS_W64_MIN_BLOCKS
 #define FLB_FS_W64_MIN_BLOCKS 3
 #endif
+// two cells per thread: four blocks of 256 threads at 64 registers (five at 48
+// spill: 2048x512 25.1 against 24.2 us per step, 4001x1201 159 against 148)
 #ifndef FLB_FS_W64X2_MIN_BLOCKS
-#define FLB_FS_W64X2_MIN_BLOCKS 5
-#endif
-#ifndef FLB_FS_QUARTER_MIN_BLOCKS
-#define FLB_FS_QUARTER_MIN_BLOCKS 4
+#define FLB_FS_W64X2_MIN_BLOCKS 4
 #endif
 // periodic index; halos of in-range tiles need one add or subtract, the
 // modulo is only reached on grids narrower than a tile
@@ -208,6 +200,7 @@ struct FlagMasks {
   uint32_t p7[kR][kW];     // after FS_2: GAS_INTERFACE bit
   uint32_t anyig[kR][kW];  // FS_3: a neighbour is IG (after FS_2)
   uint32_t cnt[kR][kW];    // after FS_4's conversion: counted by FS_4's neighbour count
+  uint8_t raw[kR * kW][32];  // the flag bytes
 };
 
 // 8-neighbourhood of bit i of word c, row r, of mask m (missing words read 0).
@@ -282,8 +275,12 @@ __device__ __forceinline__ void fs4_own_load(const KParams& p, uint32_t idx, Fs4
   o.old = p.flags_out[idx];
   o.m = static_cast<const M*>(p.mass)[idx];
   o.rho = static_cast<const C*>(p.rho)[idx];
-  // the old excess is compared only by a gas cell that stays gas (write
-  // skipping), so only a cell with the gas bit reads it
+}
+// The old excess is compared only by a gas cell that stays gas (write
+// skipping), so only a cell with the gas bit reads it; on its own, after the
+// window's loads: it waits for the flag, and they must not.
+template <class C, class M>
+__device__ __forceinline__ void fs4_own_excess(const KParams& p, uint32_t idx, Fs4Own<C, M>& o) {
   o.ex = (o.f0 & kGas) ? static_cast<const M*>(p.excess)[idx] : M(0);
 }
 
@@ -448,19 +445,15 @@ __device__ __forceinline__ void fs234_stages(const KParams& p, FlagMasks<TW>& sm
                                              int tid) {
   constexpr int kW = FlagMasks<TW>::kW, kR = FlagMasks<TW>::kR, kRW = kR * kW;
   const int lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-  for (int k = 0; k < kIters; k++) {
-    const int rw = warp + k * kWarps;  // the same for the whole warp
-    if (rw >= kRW) break;
+  auto ballots = [&](int rw, uint8_t f) {  // rw: the same for the whole warp
     const int r = rw / kW, c = rw % kW;
-    const uint8_t f = fv[k];
     // ballots of the flag bits; the masks a row needs are formed from them:
     // the outer halo rows only feed FS_2's IF dilation, the next rows also
     // FS_2's rewrite, the inner ten rows everything (warp-uniform branches)
     const uint32_t bF = __ballot_sync(0xffffffffu, (f & kFluid) != 0);
     const uint32_t bI = __ballot_sync(0xffffffffu, (f & kInterface) != 0);
     if (lane == 0) sm.a[r][c] = bF & bI;
-    if (r == 0 || r == kR - 1) continue;
+    if (r == 0 || r == kR - 1) return;
     const uint32_t bG = __ballot_sync(0xffffffffu, (f & kGas) != 0);
     const uint32_t bGI = __ballot_sync(0xffffffffu, (f & kGasInterface) != 0);
     if (lane == 0) {
@@ -469,7 +462,7 @@ __device__ __forceinline__ void fs234_stages(const KParams& p, FlagMasks<TW>& sm
       sm.gi[r][c] = bGI;
       sm.it[r][c] = bI;
     }
-    if (r == 1 || r == kR - 2) continue;
+    if (r == 1 || r == kR - 2) return;
     const uint32_t bIn = __ballot_sync(0xffffffffu, (f & kInlet) != 0);
     const uint32_t bSk = __ballot_sync(0xffffffffu, (f & (kWall | kMovingWall | kInlet)) != 0);
     if (lane == 0) {
@@ -477,6 +470,21 @@ __device__ __forceinline__ void fs234_stages(const KParams& p, FlagMasks<TW>& sm
       sm.fb[r][c] = bF;
       sm.sk[r][c] = bSk;
     }
+  };
+  if constexpr (kWarps >= 16) {
+    // one cell per thread (small grids): through shared memory (each lane its
+    // own bytes), so that the ballots are a loop; there this code runs once per
+    // block, and unrolled it takes longer to fetch than to run (101x101 14.7 ->
+    // 14.3 us per step; with two cells per thread 2048x512 24.0 -> 24.3)
+#pragma unroll
+    for (int k = 0; k < kIters; k++)
+      if (warp + k * kWarps < kRW) sm.raw[warp + k * kWarps][lane] = fv[k];
+#pragma unroll 1
+    for (int rw = warp; rw < kRW; rw += kWarps) ballots(rw, sm.raw[rw][lane]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < kIters; k++)
+      if (warp + k * kWarps < kRW) ballots(warp + k * kWarps, fv[k]);
   }
   __syncthreads();
   // FS_2 on rows 1 .. kR-2: next to an IF cell, IG -> I and G -> GI
@@ -512,10 +520,9 @@ __device__ __forceinline__ void fs234_stages(const KParams& p, FlagMasks<TW>& sm
 // one 32-cell word on either side: all that the three stencils reach), one
 // byte per lane and row-word, with the kWarps warps of the block; a window
 // inside the grid is addressed directly, one that crosses an edge wraps
-// (periodic).  Returns whether one of this lane's bytes has a gas,
-// interface or gas-interface bit.
+// (periodic).
 template <int TW, int kWarps, int kIters>
-__device__ __forceinline__ bool load_window(const KParams& p, int tx, int ty, int tid, uint8_t (&fv)[kIters]) {
+__device__ __forceinline__ void load_window(const KParams& p, int tx, int ty, int tid, uint8_t (&fv)[kIters]) {
   constexpr int kTX = TW, kW = FlagMasks<TW>::kW, kR = FlagMasks<TW>::kR, kRW = kR * kW;
   static_assert(kIters * kWarps >= kRW, "window: too few loads");
   const int nx = (int)p.nx, ny = (int)p.ny;
@@ -525,7 +532,6 @@ __device__ __forceinline__ bool load_window(const KParams& p, int tx, int ty, in
   const int wx0 = tx * kTX - 32, wy0 = ty * kTY - kHalo;
   const bool inner = wx0 >= 0 && wx0 + 32 * kW <= nx && wy0 >= 0 && wy0 + kR <= ny;
   const uint8_t* wbase = flags + (inner ? xw + wy0 * nx : 0);
-  bool nq = false;
 #pragma unroll
   for (int k = 0; k < kIters; k++) {
     const int rw = warp + k * kWarps;
@@ -534,9 +540,6 @@ __device__ __forceinline__ bool load_window(const KParams& p, int tx, int ty, in
             : inner   ? wbase[r * nx + 32 * c]
                       : flags[wrapi(xw + 32 * c, nx) + wrapi(wy0 + r, ny) * nx];
   }
-#pragma unroll
-  for (int k = 0; k < kIters; k++) nq |= (fv[k] & (kGas | kInterface | kGasInterface)) != 0;
-  return nq;
 }
 
 // One TW x 8 tile (tile coordinates tx, ty) with the TW*8/CPT threads of the
@@ -566,7 +569,15 @@ __device__ __forceinline__ uint32_t fs234_tile(const KParams& p, int tx, int ty,
   // loaded first, so the loads of all its row-words are in flight together
   constexpr int kRW = kR * kW, kIters = (kRW + kWarps - 1) / kWarps;
   uint8_t fv[kIters];
-  const bool nq = load_window<TW, kWarps, kIters>(p, tx, ty, tid, fv);
+  load_window<TW, kWarps, kIters>(p, tx, ty, tid, fv);
+#pragma unroll
+  for (int k = 0; k < CPT; k++) {
+    const int gy = ty * kTY + ly0 + k * kRowStep;
+    if (gx < nx && gy < ny) fs4_own_excess<C, M>(p, (uint32_t)gx + (uint32_t)gy * (uint32_t)nx, own[k]);
+  }
+  bool nq = false;
+#pragma unroll
+  for (int k = 0; k < kIters; k++) nq |= (fv[k] & (kGas | kInterface | kGasInterface)) != 0;
   // a quiet tile (no gas, interface or gas-interface cell in the window)
   // needs none of the masks: FS_2 and FS_3 change no flag there and FS_4
   // converts none, and each cell counts its neighbours itself
@@ -630,8 +641,7 @@ __device__ __forceinline__ void append_next(const NextLists& nl, uint32_t t, uin
 // The flag pass over one super-tile t (its kSTW / TW tiles in turn) with the
 // TW*kTY/CPT threads of the block; every thread of the block must call it.
 // Records the super-tile's activity word in nz[t] (whose previous value, the
-// word of the last step, it reads first) and appends to the next step's
-// lists.  wact_sm: one word per warp of the block.
+// word of the last step, it reads first) and appends to the next step's lists.  wact_sm: one word per warp of the block.
 template <class S, class C, class M, bool ODD, int TW, int CPT = 1>
 __device__ __forceinline__ void fs234_super_tile(const KParams& p, uint32_t t, uint32_t nsx, uint32_t* nz,
                                                  const NextLists& nl, FlagMasks<TW>& sm, uint32_t* wact_sm) {
@@ -655,8 +665,7 @@ __device__ __forceinline__ void fs234_super_tile(const KParams& p, uint32_t t, u
   if ((tid & 31) == 0) wact_sm[tid >> 5] = act;
   __syncthreads();
   if (tid < 32) {
-    uint32_t m = 0;
-    for (int w = 0; w < kWarps; w++) m |= wact_sm[w];
+    const uint32_t m = __reduce_or_sync(0xffffffffu, tid < kWarps ? wact_sm[tid] : 0u);
     if (tid == 0) nz[t] = m;
     append_next(nl, t, m, word, (uint32_t)tid);
   }

@@ -8,39 +8,35 @@
 
 namespace flb {
 
-// FS_1 on the listed super-tiles, one row of a super-tile per warp.
-// FS_1 blocks: kFs1Block threads (512: two cells per thread and super-tile,
-// x and x + 64 of a row; 1024: one cell per thread), FLB_FS1_MIN_BLOCKS per
-// SM.  Measured on a B200 (dam break, step time at 2048x512 / FS_1 time at
-// 8192x2048): 512 threads, two blocks per SM (64 registers) 28.4 / 83 us;
-// 1024 threads at 32 registers 33.3 / 103 us and at 64 registers 29.8 /
-// 93 us; 512 threads at 40 registers 33.1 / 90 us (the spills cost more than
-// the added warps gain).
-#ifndef FLB_FS1_BLOCK
-#define FLB_FS1_BLOCK 512
-#endif
-#ifndef FLB_FS1_MIN_BLOCKS
-#define FLB_FS1_MIN_BLOCKS 2
-#endif
-constexpr int kFs1Block = FLB_FS1_BLOCK;
+// FS_1 on the listed super-tiles, one row of a super-tile per warp, at 64
+// registers and 1024 threads per SM in either form: two cells per thread
+// (256-thread blocks, four per SM) takes about 500 listed super-tiles in one
+// round; with one cell per thread (512 x 2) the pass is shorter where there are
+// few.  Measured on a B200, us per step with two | one (the flag pass
+// likewise): 101x101 17.2 | 14.9, 300x120 16.4 | 15.0, 1001x401 26.3 | 25.4,
+// 2048x512 24.2 | 27.6, 8192x2048 232 | 264.  The line is kSmallTiles.
+constexpr int kFs1Block = 256;   // two cells per thread (x and x + 32 of a row), four blocks per SM
+constexpr int kFs1Small = 512;   // one cell per thread, two blocks per SM
 // lc: the next step's list lengths and marks, cleared here for this step's
 // flag pass.
-template <class S, class C, class M, bool HW, bool ODD>
-__global__ void __launch_bounds__(kFs1Block, FLB_FS1_MIN_BLOCKS) k_fs1(const __grid_constant__ KParams p,
+template <class S, class C, class M, bool HW, bool ODD, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_fs1(const __grid_constant__ KParams p,
                                                                        const TileList tl, const ListClear lc) {
   pdl_wait();
   pdl_trigger();
   clear_next_lists(lc);
-  constexpr uint32_t kCpr = kFs1Block / 32 / kSTH;     // warps per row of a super-tile
+  constexpr uint32_t kCpr = BLOCK / 32 / kSTH;         // warps per row of a super-tile
   constexpr uint32_t kCells = kSTW / (32u * kCpr);     // cells per thread and super-tile
   static_assert(kCells * 32u * kCpr == kSTW && kCells <= 2u, "FS_1: one or two cells per thread and super-tile");
-  static_assert(kFs1Block >= 118, "FS_1: prefetch_super_tile needs 118 threads");
+  static_assert(BLOCK >= 118, "FS_1: prefetch_super_tile needs 118 threads");
+  // the block's first entry is loaded with the length (the list holds at least
+  // a grid of entries, whatever its length)
+  uint32_t t = tile_at(tl, blockIdx.x);
   const uint32_t n = tile_count(tl);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t row = warp % kSTH, chunk = warp / kSTH;
   const uint32_t nx = p.nx;
-  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-    const uint32_t t = tile_at(tl, i);
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x, t = i < n ? tile_at(tl, i) : 0u) {
     // the block's next super-tile into L2 while this one is worked on
     if (i + gridDim.x < n) prefetch_super_tile(p, tile_at(tl, i + gridDim.x), tl.nsx, sizeof(S), true, sizeof(M));
     const uint32_t y = (t / tl.nsx) * kSTH + row;
@@ -92,9 +88,7 @@ __global__ void k_apply_recon(const __grid_constant__ KParams p, uint32_t odd) {
 // TW x 8 tiles, CPT cells per thread.
 template <int TW, int CPT>
 constexpr int fs234_min_blocks() {
-  return TW == 128  ? (CPT == 1 ? FLB_FS_WIDE_MIN_BLOCKS : CPT == 2 ? FLB_FS_HALF_MIN_BLOCKS : FLB_FS_QUARTER_MIN_BLOCKS)
-         : TW == 64 ? (CPT == 1 ? FLB_FS_W64_MIN_BLOCKS : FLB_FS_W64X2_MIN_BLOCKS)
-                    : 6;
+  return TW == 64 ? (CPT == 1 ? FLB_FS_W64_MIN_BLOCKS : FLB_FS_W64X2_MIN_BLOCKS) : 6;
 }
 template <class S, class C, class M, bool ODD, int TW, int CPT>
 __global__ void __launch_bounds__(TW* kTY / CPT, fs234_min_blocks<TW, CPT>())
@@ -113,13 +107,14 @@ __global__ void __launch_bounds__(TW* kTY / CPT, fs234_min_blocks<TW, CPT>())
 // ---- launchers -------------------------------------------------------------------
 template <class S, class C, class M>
 void launch_fs1(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const TileList& tl, uint32_t grid,
-                const ListClear& lc) {
-  if (hw) {
-    if (odd) launch_pdl(k_fs1<S, C, M, true, true>, grid, kFs1Block, st, kp, tl, lc);
-    else launch_pdl(k_fs1<S, C, M, true, false>, grid, kFs1Block, st, kp, tl, lc);
+                const ListClear& lc, bool one_cell) {
+  const KParams q = as_even(kp, odd);
+  if (one_cell) {
+    if (hw) launch_pdl(k_fs1<S, C, M, true, false, kFs1Small>, grid, kFs1Small, st, q, tl, lc);
+    else launch_pdl(k_fs1<S, C, M, false, false, kFs1Small>, grid, kFs1Small, st, q, tl, lc);
   } else {
-    if (odd) launch_pdl(k_fs1<S, C, M, false, true>, grid, kFs1Block, st, kp, tl, lc);
-    else launch_pdl(k_fs1<S, C, M, false, false>, grid, kFs1Block, st, kp, tl, lc);
+    if (hw) launch_pdl(k_fs1<S, C, M, true, false, kFs1Block>, grid, kFs1Block, st, q, tl, lc);
+    else launch_pdl(k_fs1<S, C, M, false, false, kFs1Block>, grid, kFs1Block, st, q, tl, lc);
   }
 }
 
@@ -138,13 +133,9 @@ template <class S, class C, class M, int TW, int CPT>
 void launch_fs234_form(const KParams& kp, cudaStream_t st, uint32_t odd, const TileList& tl, uint32_t grid,
                        uint32_t* nz, const NextLists& nl) {
   constexpr int threads = TW * kTY / CPT;
-  if (tl.ntiles <= kWideTiles) {
-    if (odd) launch_pdl(k_fs234<S, C, M, true, TW, CPT>, grid, threads, st, kp, tl, nz, nl);
-    else launch_pdl(k_fs234<S, C, M, false, TW, CPT>, grid, threads, st, kp, tl, nz, nl);
-  } else {
-    if (odd) k_fs234<S, C, M, true, TW, CPT><<<grid, threads, 0, st>>>(kp, tl, nz, nl);
-    else k_fs234<S, C, M, false, TW, CPT><<<grid, threads, 0, st>>>(kp, tl, nz, nl);
-  }
+  const KParams q = as_even(kp, odd);
+  if (tl.ntiles <= kWideTiles) launch_pdl(k_fs234<S, C, M, false, TW, CPT>, grid, threads, st, q, tl, nz, nl);
+  else k_fs234<S, C, M, false, TW, CPT><<<grid, threads, 0, st>>>(q, tl, nz, nl);
 }
 
 template <class S, class C, class M>
@@ -152,11 +143,8 @@ int launch_fs234(const KParams& kp, cudaStream_t st, uint32_t odd, const TileLis
                  const NextLists& nl, int form) {
   switch (form) {
     case FS_FORM_W32: launch_fs234_form<S, C, M, 32, 1>(kp, st, odd, tl, grid, nz, nl); break;
-    case FS_FORM_W128X2: launch_fs234_form<S, C, M, 128, 2>(kp, st, odd, tl, grid, nz, nl); break;
-    case FS_FORM_W128X4: launch_fs234_form<S, C, M, 128, 4>(kp, st, odd, tl, grid, nz, nl); break;
     case FS_FORM_W64X1: launch_fs234_form<S, C, M, 64, 1>(kp, st, odd, tl, grid, nz, nl); break;
-    case FS_FORM_W64X2: launch_fs234_form<S, C, M, 64, 2>(kp, st, odd, tl, grid, nz, nl); break;
-    default: launch_fs234_form<S, C, M, 128, 1>(kp, st, odd, tl, grid, nz, nl); break;
+    default: launch_fs234_form<S, C, M, 64, 2>(kp, st, odd, tl, grid, nz, nl); break;
   }
   return 1;
 }
@@ -172,19 +160,19 @@ int fs234_blocks_per_sm() {
 template <class S, class C, class M>
 int fs_blocks_per_sm(int which, int form) {
   int n = 0;
-  if (which == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_fs1<S, C, M, true, false>, kFs1Block, 0);
+  if (which == 0 && form == 1)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_fs1<S, C, M, true, false, kFs1Small>, kFs1Small, 0);
+  else if (which == 0)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_fs1<S, C, M, true, false, kFs1Block>, kFs1Block, 0);
   else if (form == FS_FORM_W32) n = fs234_blocks_per_sm<S, C, M, 32, 1>();
-  else if (form == FS_FORM_W128X2) n = fs234_blocks_per_sm<S, C, M, 128, 2>();
-  else if (form == FS_FORM_W128X4) n = fs234_blocks_per_sm<S, C, M, 128, 4>();
   else if (form == FS_FORM_W64X1) n = fs234_blocks_per_sm<S, C, M, 64, 1>();
-  else if (form == FS_FORM_W64X2) n = fs234_blocks_per_sm<S, C, M, 64, 2>();
-  else n = fs234_blocks_per_sm<S, C, M, 128, 1>();
+  else n = fs234_blocks_per_sm<S, C, M, 64, 2>();
   return n > 0 ? n : 1;
 }
 
 #define FLB_INSTANTIATE(S, C, M)                                                                                  \
   template void launch_fs1<S, C, M>(const KParams&, cudaStream_t, uint32_t, bool, const TileList&, uint32_t,       \
-                                    const ListClear&);                                                          \
+                                    const ListClear&, bool);                                                     \
   template void launch_apply_recon<S, C, M>(const KParams&, cudaStream_t, uint32_t);                             \
   template int launch_fs234<S, C, M>(const KParams&, cudaStream_t, uint32_t, const TileList&, uint32_t, uint32_t*,   \
                                      const NextLists&, int);                                                     \

@@ -7,7 +7,7 @@
 // break) every pass is a single round of latency-bound work, and the launch,
 // ramp-up and drain of each kernel are a large part of the step.  Here one
 // cooperative launch runs an even number of steps: every CTA stays resident
-// (one per SM, 1024 threads, one cell per thread of a 128x8 super-tile), and
+// (two per SM, 512 threads, one cell per thread of a 64x8 super-tile), and
 // the three passes of each step are separated by grid barriers in global
 // memory instead of kernel boundaries.  The passes themselves are the same
 // device code as the per-pass kernels (fs1_cell, sc_cell, fs234_super_tile),
@@ -23,7 +23,7 @@
 namespace flb {
 namespace {
 
-constexpr int kPBlock = 1024;
+constexpr int kPBlock = 512;
 
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* a) {
   uint32_t v;
@@ -82,43 +82,43 @@ __device__ __forceinline__ bool next_barrier(const FspArgs& a, uint32_t& nbar, i
   return good;
 }
 
-// One time step with parity ODD (p: the step's parameters, its flag buffers
-// in the order of that parity).  Returns false when a barrier gave up.
-template <class S, class C, class M, bool HW, bool FU, bool ODD>
-__device__ __forceinline__ bool fsp_step(const KParams& p, const FspArgs& a, FlagMasks<128>& sm, uint32_t* wact_sm,
+// One time step of parity `odd` (p: the step's parameters, its flag buffers in
+// the order of that parity, its slots as of an even step: as_even).  Returns false when a barrier gave up.
+template <class S, class C, class M, bool HW, bool FU>
+__device__ __forceinline__ bool fsp_step(const KParams& p, const uint32_t odd, const FspArgs& a, FlagMasks<64>& sm, uint32_t* wact_sm,
                                          uint32_t& nbar, int& ok) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t row = warp % kSTH, xo = (warp / kSTH) * 32u + lane;  // this thread's cell of a super-tile
   const uint32_t G = gridDim.x;
-  const uint32_t* lsc = a.list[ODD][0];
-  const uint32_t* lfs = a.list[ODD][1];
+  const uint32_t* lsc = a.list[odd][0];
+  const uint32_t* lfs = a.list[odd][1];
   // lengths of this step's lists (built by the previous step)
   const uint32_t T = a.nsx * a.nsy;
-  const uint32_t nsc = min(__ldcg(a.lcount + 2 * ODD), T);
-  const uint32_t nfs = a.fs_all ? T : min(__ldcg(a.lcount + 2 * ODD + 1), T);
+  const uint32_t nsc = min(__ldcg(a.lcount + 2 * odd), T);
+  const uint32_t nfs = a.fs_all ? T : min(__ldcg(a.lcount + 2 * odd + 1), T);
   // the next step's list lengths and marks, which this step's flag pass
   // appends to (the previous step's passes have finished reading them)
-  clear_next_lists(ListClear{a.lcount + 2 * (ODD ^ 1), a.lbits + (ODD ^ 1) * a.nwords, a.nwords});
+  clear_next_lists(ListClear{a.lcount + 2 * (odd ^ 1u), a.lbits + (odd ^ 1u) * a.nwords, a.nwords});
   // FS_1: mass exchange and gas reconstruction
   for (uint32_t i = blockIdx.x; i < nsc; i += G) {
     const uint32_t t = __ldcg(lsc + i);
     const uint32_t y = (t / a.nsx) * kSTH + row, x = (t % a.nsx) * kSTW + xo;
-    if (y < p.ny && x < p.nx) fs1_cell<S, C, M, HW, ODD>(p, x, y);
+    if (y < p.ny && x < p.nx) fs1_cell<S, C, M, HW, false>(p, x, y);
   }
   if (!next_barrier(a, nbar, ok)) return false;
   // stream-collide
   for (uint32_t i = blockIdx.x; i < nsc; i += G) {
     const uint32_t t = __ldcg(lsc + i);
     const uint32_t y = (t / a.nsx) * kSTH + row, x = (t % a.nsx) * kSTW + xo;
-    if (y < p.ny && x < p.nx) sc_cell<S, C, M, true, HW, true, ODD, FU>(p, x, y);
+    if (y < p.ny && x < p.nx) sc_cell<S, C, M, true, HW, true, false, FU>(p, x, y);
   }
   if (!next_barrier(a, nbar, ok)) return false;
   // FS_2..4: flag stencil, mass / excess / fill level, activity words and the
   // next step's lists
-  const NextLists nl{a.list[ODD ^ 1][0], a.list[ODD ^ 1][1], a.lcount + 2 * (ODD ^ 1), a.lbits + (ODD ^ 1) * a.nwords,
+  const NextLists nl{a.list[odd ^ 1u][0], a.list[odd ^ 1u][1], a.lcount + 2 * (odd ^ 1u), a.lbits + (odd ^ 1u) * a.nwords,
                      a.nsx, a.nsy};
   for (uint32_t i = blockIdx.x; i < nfs; i += G)
-    fs234_super_tile<S, C, M, ODD, 128>(p, a.fs_all ? i : __ldcg(lfs + i), a.nsx, a.nz, nl, sm, wact_sm);
+    fs234_super_tile<S, C, M, false, 64>(p, a.fs_all ? i : __ldcg(lfs + i), a.nsx, a.nz, nl, sm, wact_sm);
   return next_barrier(a, nbar, ok);
 }
 
@@ -126,10 +126,10 @@ __device__ __forceinline__ bool fsp_step(const KParams& p, const FspArgs& a, Fla
 // parameters of the even steps (flags = buffer 0, flags_out = buffer 1), p1
 // those of the odd steps (swapped).
 template <class S, class C, class M, bool HW, bool FU>
-__global__ void __launch_bounds__(kPBlock, 1) k_fs_persist(const __grid_constant__ KParams p0,
+__global__ void __launch_bounds__(kPBlock, 2) k_fs_persist(const __grid_constant__ KParams p0,
                                                           const __grid_constant__ KParams p1,
                                                           const __grid_constant__ FspArgs a) {
-  __shared__ FlagMasks<128> sm;
+  __shared__ FlagMasks<64> sm;
   __shared__ uint32_t wact_sm[kPBlock / 32];
   __shared__ int ok;
   // a barrier of an earlier launch gave up: the state is undefined until the
@@ -139,10 +139,9 @@ __global__ void __launch_bounds__(kPBlock, 1) k_fs_persist(const __grid_constant
   if (!ok) return;
   if (a.trace && blockIdx.x == 0 && threadIdx.x == 0) a.trace[0] = global_ns();
   uint32_t nbar = 0;
-  for (uint32_t s = 0; s < a.steps; s += 2) {
-    if (!fsp_step<S, C, M, HW, FU, false>(p0, a, sm, wact_sm, nbar, ok)) return;
-    if (!fsp_step<S, C, M, HW, FU, true>(p1, a, sm, wact_sm, nbar, ok)) return;
-  }
+#pragma unroll 1
+  for (uint32_t s = 0; s < a.steps; s++)
+    if (!fsp_step<S, C, M, HW, FU>(s & 1u ? p1 : p0, s & 1u, a, sm, wact_sm, nbar, ok)) return;
 }
 
 template <class S, class C, class M>
@@ -171,7 +170,7 @@ cudaError_t launch_fs_persist(const KParams& p0, const KParams& p1, const FspArg
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, pick_fsp<S, C, M>(hw, fu), p0, p1, a);
+  return cudaLaunchKernelEx(&cfg, pick_fsp<S, C, M>(hw, fu), p0, as_even(p1, 1u), a);
 }
 
 template <class S, class C, class M>

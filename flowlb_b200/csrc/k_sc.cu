@@ -53,9 +53,19 @@ __global__ void __launch_bounds__(kBlock, FLB_SC_MIN_BLOCKS) k_sc_scalar(const _
   sc_cell<S, C, M, FS, HW, WM, ODD, FU>(p, x, y);
 }
 
-// Free surface: the listed super-tiles, one row of a super-tile per warp.
-template <class S, class C, class M, bool HW, bool ODD, bool FU>
-__global__ void __launch_bounds__(kListBlock, 2048 / kListBlock) k_sc_list(const __grid_constant__ KParams p,
+// Free surface: the listed super-tiles, one row of 32 cells per warp, BLOCK
+// threads, MB blocks resident per SM.  Measured on a B200, us per step of the
+// dam break (grid, storage: 512 threads x 4 at 32 registers | 512 x 2 at 64 |
+// 256 x 4 at 64, two cells per thread):
+//   601x301 F32, reference arithmetic  19.5 | 16.0 | 18.1
+//   1001x401 F32  24.8 | 22.8 | 24.4       2048x512 F32  24.3 | 24.0 | 23.7
+//   2048x512 F64  32.0 | 28.4 | 27.6       8192x2048 F32  233 | 242 | 238
+// So: 512 x 2 while the blocks are about one round (kScSmallTiles), 512 x 4
+// where FP32 with the fused arithmetic (few spills at 32 registers) is bound by
+// memory (more than kScLargeTiles super-tiles), 256 x 4 elsewhere.
+constexpr uint32_t kScSmallTiles = 1024, kScLargeTiles = 8192;
+template <class S, class C, class M, bool HW, bool ODD, bool FU, int BLOCK, int MB>
+__global__ void __launch_bounds__(BLOCK, MB) k_sc_list(const __grid_constant__ KParams p,
                                                                            const TileList tl) {
   // the list was built two kernels back (FS_1 waited for it), so it is read
   // before waiting for FS_1, whose writes the cell updates need
@@ -135,10 +145,11 @@ __device__ __forceinline__ void load_bytes(const uint8_t* ptr, uint8_t (&f)[V]) 
 constexpr int kVecBlock = 256;
 
 // V consecutive cells x0 .. x0+V-1 of row y per thread (x0 a multiple of V;
-// the 32 lanes of the warp take consecutive groups of one row, every lane of
-// the warp must call it).  Used over whole rows (k_sc_vec) and over the rows
+// LPR consecutive lanes of the warp, `lane` the position among them, take
+// consecutive groups of one row; every lane of the warp must call it, with x0
+// past the row's end where it has no cells).  Used over whole rows (k_sc_vec) and over the rows
 // of listed super-tiles (k_sc_list_vec).
-template <class S, class C, class M, bool FS, bool HW, bool WM, bool ODD, bool FU>
+template <class S, class C, class M, bool FS, bool HW, bool WM, bool ODD, bool FU, uint32_t LPR = 32u>
 __device__ __forceinline__ void sc_vec_cells(const KParams& p, uint32_t x0, uint32_t y, uint32_t lane) {
   constexpr int V = Lanes<S>::V;
   constexpr bool DEV = kDev<S, FS, FU>;
@@ -148,7 +159,7 @@ __device__ __forceinline__ void sc_vec_cells(const KParams& p, uint32_t x0, uint
   const uint32_t row = y * nx;
   const uint32_t rowu = (y + 1u == ny ? 0u : y + 1u) * nx;
   const uint32_t rowd = (y == 0u ? ny - 1u : y - 1u) * nx;
-  const bool tail = (lane == 31u) || (x0 + V >= nx);  // the cell past this lane is not the next lane's
+  const bool tail = (lane == LPR - 1u) || (x0 + V >= nx);  // the cell past this lane is not the next lane's
   const uint32_t xn = (x0 + V >= nx) ? 0u : x0 + V;   // position past this lane (periodic wrap)
   if (DEV && x0 == 0 && y == 0) p.tstep[!ODD] = p.tstep[ODD] + 1u;
 
@@ -292,28 +303,27 @@ __global__ void __launch_bounds__(kVecBlock, FU ? (std::is_same<S, __half>::valu
 }
 
 // Free surface, vector data path: the listed super-tiles, each row of a
-// super-tile taken by kSTW / (32 V) warps (one warp for FP32 and FP16S).
+// super-tile taken by kSTW / V lanes (half a warp for FP32 and FP16S).
 template <class S>
 __host__ __device__ constexpr int list_vec_block() {
-  return (int)kSTH * (int)(kSTW / (32u * (uint32_t)Lanes<S>::V)) * 32;
+  return (int)(kSTH * kSTW / (uint32_t)Lanes<S>::V);
 }
 template <class S, class C, class M, bool HW, bool ODD, bool FU>
 __global__ void __launch_bounds__(list_vec_block<S>(), 1024 / list_vec_block<S>())
     k_sc_list_vec(const __grid_constant__ KParams p, const TileList tl) {
-  constexpr uint32_t V = (uint32_t)Lanes<S>::V, wpr = kSTW / (32u * V);
+  constexpr uint32_t V = (uint32_t)Lanes<S>::V, LPR = kSTW / V;
+  static_assert(LPR <= 32u, "a row of a super-tile within one warp");
   // the list was built two kernels back (FS_1 waited for it), so it is read
   // before waiting for FS_1, whose writes the cell updates need
   const uint32_t n = tile_count(tl);
   pdl_wait();
   pdl_trigger();
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t row = warp / wpr, chunk = warp % wpr;
+  const uint32_t lane = threadIdx.x % LPR, row = threadIdx.x / LPR;
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
     const uint32_t t = tile_at(tl, i);
     const uint32_t y = (t / tl.nsx) * kSTH + row;
-    if (y >= p.ny) continue;  // warp-uniform
-    const uint32_t x0 = (t % tl.nsx) * kSTW + (chunk * 32u + lane) * V;
-    sc_vec_cells<S, C, M, true, HW, true, ODD, FU>(p, x0, y, lane);
+    const uint32_t x0 = y < p.ny ? (t % tl.nsx) * kSTW + lane * V : p.nx;
+    sc_vec_cells<S, C, M, true, HW, true, ODD, FU, LPR>(p, x0, y < p.ny ? y : 0u, lane);
   }
 }
 
@@ -625,24 +635,22 @@ int vec_width(int precision) {
 template <class S, class C, class M, bool FU>
 static void launch_sc_list_f(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const TileList& tl,
                              uint32_t grid, bool vec) {
+  const KParams q = as_even(kp, odd);
   if (vec) {
     constexpr int B = list_vec_block<S>();
-    if (hw) {
-      if (odd) launch_pdl(k_sc_list_vec<S, C, M, true, true, FU>, grid, B, st, kp, tl);
-      else launch_pdl(k_sc_list_vec<S, C, M, true, false, FU>, grid, B, st, kp, tl);
-    } else {
-      if (odd) launch_pdl(k_sc_list_vec<S, C, M, false, true, FU>, grid, B, st, kp, tl);
-      else launch_pdl(k_sc_list_vec<S, C, M, false, false, FU>, grid, B, st, kp, tl);
-    }
+    if (hw) launch_pdl(k_sc_list_vec<S, C, M, true, false, FU>, grid, B, st, q, tl);
+    else launch_pdl(k_sc_list_vec<S, C, M, false, false, FU>, grid, B, st, q, tl);
     return;
   }
-  if (hw) {
-    if (odd) launch_pdl(k_sc_list<S, C, M, true, true, FU>, grid, kListBlock, st, kp, tl);
-    else launch_pdl(k_sc_list<S, C, M, true, false, FU>, grid, kListBlock, st, kp, tl);
-  } else {
-    if (odd) launch_pdl(k_sc_list<S, C, M, false, true, FU>, grid, kListBlock, st, kp, tl);
-    else launch_pdl(k_sc_list<S, C, M, false, false, FU>, grid, kListBlock, st, kp, tl);
-  }
+  auto go = [&](auto block, auto mb) {
+    constexpr int BLOCK = decltype(block)::value, MB = decltype(mb)::value;
+    if (hw) launch_pdl(k_sc_list<S, C, M, true, false, FU, BLOCK, MB>, grid, BLOCK, st, q, tl);
+    else launch_pdl(k_sc_list<S, C, M, false, false, FU, BLOCK, MB>, grid, BLOCK, st, q, tl);
+  };
+  using std::integral_constant;
+  if (tl.ntiles <= kScSmallTiles) go(integral_constant<int, 512>{}, integral_constant<int, 2>{});
+  else if (FU && sizeof(C) == 4 && tl.ntiles > kScLargeTiles) go(integral_constant<int, 512>{}, integral_constant<int, 4>{});
+  else go(integral_constant<int, 256>{}, integral_constant<int, 4>{});
 }
 
 template <class S, class C, class M>
@@ -653,17 +661,11 @@ void launch_sc_list(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, c
 }
 
 template <class S, class C, class M>
-int sc_list_blocks_per_sm(bool vec) {
+int sc_list_blocks_per_sm(bool vec, uint32_t ntiles) {
+  if (!vec) return ntiles <= kScSmallTiles ? 2 : 4;  // the launch bounds
   int n = 0, m = 0;
-  if (vec) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sc_list_vec<S, C, M, true, false, false>,
-                                                  list_vec_block<S>(), 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_sc_list_vec<S, C, M, true, false, true>,
-                                                  list_vec_block<S>(), 0);
-  } else {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sc_list<S, C, M, true, false, false>, kListBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_sc_list<S, C, M, true, false, true>, kListBlock, 0);
-  }
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sc_list_vec<S, C, M, true, false, false>, list_vec_block<S>(), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_sc_list_vec<S, C, M, true, false, true>, list_vec_block<S>(), 0);
   n = n < m ? n : m;
   return n > 0 ? n : 1;
 }
@@ -672,7 +674,7 @@ int sc_list_blocks_per_sm(bool vec) {
   template void launch_sc<S, C, M>(const KParams&, cudaStream_t, uint32_t, bool, bool, bool, bool, bool);     \
   template void launch_sc_list<S, C, M>(const KParams&, cudaStream_t, uint32_t, bool, const TileList&, uint32_t,  \
                                         bool, bool);                                                            \
-  template int sc_list_blocks_per_sm<S, C, M>(bool);
+  template int sc_list_blocks_per_sm<S, C, M>(bool, uint32_t);
 FLB_FOR_EACH_VARIANT(FLB_INSTANTIATE)
 #undef FLB_INSTANTIATE
 

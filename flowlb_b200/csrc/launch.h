@@ -42,13 +42,13 @@ template <class S, class C, class M>
 void launch_sc_list(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const TileList& tl, uint32_t grid,
                     bool fu, bool vec);
 template <class S, class C, class M>
-int sc_list_blocks_per_sm(bool vec);
+int sc_list_blocks_per_sm(bool vec, uint32_t ntiles);
 
 // FS_1 (clears the next step's list lengths), its reference-mode apply, and
 // FS_2..4 on listed super-tiles (appends the next step's lists)
 template <class S, class C, class M>
 void launch_fs1(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const TileList& tl, uint32_t grid,
-                const ListClear& lc);
+                const ListClear& lc, bool one_cell);
 template <class S, class C, class M>
 void launch_apply_recon(const KParams& kp, cudaStream_t st, uint32_t odd);
 template <class S, class C, class M>
@@ -56,9 +56,9 @@ int launch_fs234(const KParams& kp, cudaStream_t st, uint32_t odd, const TileLis
                  const NextLists& nl, int form);
 // launch forms of the flag pass: tile width x cells per thread (threads per
 // block = width * 8 / cells per thread)
-enum FsForm { FS_FORM_W128X1 = 0, FS_FORM_W32 = 1, FS_FORM_W128X2 = 2, FS_FORM_W128X4 = 4, FS_FORM_W64X1 = 5,
-              FS_FORM_W64X2 = 6 };
-// resident blocks per SM of FS_1 (which 0) or of the flag pass in `form` (which 1)
+enum FsForm { FS_FORM_W32 = 1, FS_FORM_W64X1 = 5, FS_FORM_W64X2 = 6 };
+// resident blocks per SM of FS_1 with `form` cells per thread (which 0) or of
+// the flag pass in `form` (which 1)
 template <class S, class C, class M>
 int fs_blocks_per_sm(int which, int form);
 
