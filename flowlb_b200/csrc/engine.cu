@@ -39,9 +39,6 @@ constexpr int kGraphPairs = 16;  // steps per large graph = 2 * kGraphPairs
 // (0 super-tiles).  (As one thread-block cluster of 16 CTAs with the hardware
 // barrier, small grids only: 64x48 13.6, 101x101 17.3 against 14.3.)
 constexpr uint32_t kPersistAutoTiles = 0;
-// Up to this many super-tiles FS_1 and the flag pass take one cell per thread
-// (k_fs.cu).
-constexpr uint32_t kSmallTiles = 1024;
 constexpr uint32_t kPersistWaitLimit = 1u << 22;  // barrier polls before the persistent step gives up
 
 struct GraphSlot {
@@ -65,7 +62,6 @@ struct flb_engine {
   bool fs = false, hw = false, has_io = false;
   bool use_vec = false;       // vectorised stream-collide (single phase)
   bool use_vec_list = false;  // vectorised listed stream-collide (free surface)
-  bool fs_one_cell = false;          // FS_1 with one cell per thread
   int fs_form = FS_FORM_W64X2;  // launch form of the flag pass (FsForm)
   bool fused = false;    // fused SRT arithmetic in stream-collide
   uint64_t t = 0;
@@ -176,7 +172,7 @@ struct Ops {
     launch_sc_list<S, C, M>(h->kp, h->stream, odd, h->hw, tl, h->grid_sc, h->fused, h->use_vec_list);
   }
   static void fs1(flb_engine* h, uint32_t odd, const TileList& tl, const ListClear& lc) {
-    launch_fs1<S, C, M>(h->kp, h->stream, odd, h->hw, tl, h->grid_fs1, lc, h->fs_one_cell);
+    launch_fs1<S, C, M>(h->kp, h->stream, odd, h->hw, tl, h->grid_fs1, lc);
   }
   static int fs234(flb_engine* h, uint32_t odd, const TileList& tl, const NextLists& nl) {
     return launch_fs234<S, C, M>(h->kp, h->stream, odd, tl, h->grid_fs234, h->d_nz, nl, h->fs_form);
@@ -185,8 +181,8 @@ struct Ops {
   // without one cost their launch: 64x48 18.2 -> 16.4 us per step)
   static void grids(flb_engine* h, int nsm) {
     h->grid_sc = std::min(h->ntiles, (uint32_t)(nsm * sc_list_blocks_per_sm<S, C, M>(h->use_vec_list, h->ntiles)));
-    h->grid_fs1 = std::min(h->ntiles, (uint32_t)(nsm * fs_blocks_per_sm<S, C, M>(0, h->fs_one_cell ? 1 : 2)));
-    h->grid_fs234 = std::min(h->ntiles, (uint32_t)(nsm * fs_blocks_per_sm<S, C, M>(1, h->fs_form)));
+    h->grid_fs1 = std::min(h->ntiles, (uint32_t)(nsm * fs1_blocks_per_sm(h->ntiles)));
+    h->grid_fs234 = std::min(h->ntiles, (uint32_t)(nsm * fs234_blocks_per_sm(h->fs_form, h->ntiles)));
   }
   static cudaError_t mt(flb_engine* h, const MtArgs& a) {
     if constexpr (std::is_same<S, float>::value && std::is_same<M, float>::value)
@@ -853,8 +849,7 @@ FLB_API flb_status flb_create(const flb_case_desc* desc, flb_handle* out) {
     // FS_1 and the flag pass: one cell per thread on grids of up to
     // kSmallTiles super-tiles, two above (FsForm, k_fs.cu).
     // FLB_FS_FLAG_FORM selects another flag-pass form, with the same results.
-    h->fs_one_cell = tiles <= kSmallTiles;
-    h->fs_form = h->fs_one_cell ? FS_FORM_W64X1 : FS_FORM_W64X2;
+    h->fs_form = tiles <= kSmallTiles ? FS_FORM_W64X1 : FS_FORM_W64X2;
     if (const char* v = std::getenv("FLB_FS_FLAG_FORM")) {
       if (!std::strcmp(v, "32")) h->fs_form = FS_FORM_W32;
       else if (!std::strcmp(v, "64x1") || !std::strcmp(v, "128x1")) h->fs_form = FS_FORM_W64X1;

@@ -142,14 +142,6 @@ constexpr int kTY = 8, kHalo = 3;
 #define FLB_FS_PDL_TILES 8192
 #endif
 constexpr uint32_t kWideTiles = FLB_FS_PDL_TILES;
-#ifndef FLB_FS_W64_MIN_BLOCKS
-#define FLB_FS_W64_MIN_BLOCKS 3
-#endif
-// two cells per thread: four blocks of 256 threads at 64 registers (five at 48
-// spill: 2048x512 25.1 against 24.2 us per step, 4001x1201 159 against 148)
-#ifndef FLB_FS_W64X2_MIN_BLOCKS
-#define FLB_FS_W64X2_MIN_BLOCKS 4
-#endif
 // periodic index; halos of in-range tiles need one add or subtract, the
 // modulo is only reached on grids narrower than a tile
 __device__ __forceinline__ int wrapi(int v, int n) {

@@ -3,6 +3,8 @@
 // flag-stencil kernel (lbmKernel2D.cu:124-303) that also lists the next
 // step's super-tiles.  The per-cell and per-tile code is in fs_cells.cuh.
 // Templated on the step parity.
+#include <type_traits>
+
 #include "fs_cells.cuh"
 #include "launch.h"
 
@@ -14,13 +16,18 @@ namespace flb {
 // round; with one cell per thread (512 x 2) the pass is shorter where there are
 // few.  Measured on a B200, us per step with two | one (the flag pass
 // likewise): 101x101 17.2 | 14.9, 300x120 16.4 | 15.0, 1001x401 26.3 | 25.4,
-// 2048x512 24.2 | 27.6, 8192x2048 232 | 264.  The line is kSmallTiles.
+// 2048x512 24.2 | 27.6, 8192x2048 232 | 264.  The line is kSmallTiles.  At 64
+// registers the FP64 mass arithmetic spills (136 bytes, FP64 storage 350); on
+// grids of up to kTinyTiles super-tiles, whose listed ones fit one block per SM,
+// the one-cell form takes 128: 300x120 14.4 -> 13.4, 601x301 16.2 -> 15.0 (but
+// 1001x401 22.8 -> 24.1; two cells at 85 registers, three blocks per SM:
+// 2048x512 23.4 -> 25.1).
 constexpr int kFs1Block = 256;   // two cells per thread (x and x + 32 of a row), four blocks per SM
-constexpr int kFs1Small = 512;   // one cell per thread, two blocks per SM
+constexpr int kFs1Small = 512;   // one cell per thread, two blocks per SM, or one
 // lc: the next step's list lengths and marks, cleared here for this step's
 // flag pass.
-template <class S, class C, class M, bool HW, bool ODD, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_fs1(const __grid_constant__ KParams p,
+template <class S, class C, class M, bool HW, bool ODD, int BLOCK, int MB>
+__global__ void __launch_bounds__(BLOCK, MB) k_fs1(const __grid_constant__ KParams p,
                                                                        const TileList tl, const ListClear lc) {
   pdl_wait();
   pdl_trigger();
@@ -85,13 +92,13 @@ __global__ void k_apply_recon(const __grid_constant__ KParams p, uint32_t odd) {
 
 // The listed super-tiles: each block runs the flag pass on a super-tile,
 // records its activity word in nz and appends to the next step's lists.
-// TW x 8 tiles, CPT cells per thread.
-template <int TW, int CPT>
-constexpr int fs234_min_blocks() {
-  return TW == 64 ? (CPT == 1 ? FLB_FS_W64_MIN_BLOCKS : FLB_FS_W64X2_MIN_BLOCKS) : 6;
-}
-template <class S, class C, class M, bool ODD, int TW, int CPT>
-__global__ void __launch_bounds__(TW* kTY / CPT, fs234_min_blocks<TW, CPT>())
+// TW x 8 tiles, CPT cells per thread, MB blocks resident per SM: with one cell
+// per thread two on grids of up to kTinyTiles super-tiles (three spill at 40
+// registers: 300x120 14.4 against 13.4 us per step with FS_1's form), three
+// above (1001x401 22.8 against 23.4); with two cells four (five spill at 48:
+// 2048x512 25.1 against 24.2, 4001x1201 159 against 148).
+template <class S, class C, class M, bool ODD, int TW, int CPT, int MB>
+__global__ void __launch_bounds__(TW* kTY / CPT, MB)
     k_fs234(const __grid_constant__ KParams p, const TileList tl, uint32_t* __restrict__ nz, const NextLists nl) {
   __shared__ FlagMasks<TW> sm;
   __shared__ uint32_t wact_sm[TW * kTY / CPT / 32];
@@ -107,15 +114,17 @@ __global__ void __launch_bounds__(TW* kTY / CPT, fs234_min_blocks<TW, CPT>())
 // ---- launchers -------------------------------------------------------------------
 template <class S, class C, class M>
 void launch_fs1(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const TileList& tl, uint32_t grid,
-                const ListClear& lc, bool one_cell) {
+                const ListClear& lc) {
   const KParams q = as_even(kp, odd);
-  if (one_cell) {
-    if (hw) launch_pdl(k_fs1<S, C, M, true, false, kFs1Small>, grid, kFs1Small, st, q, tl, lc);
-    else launch_pdl(k_fs1<S, C, M, false, false, kFs1Small>, grid, kFs1Small, st, q, tl, lc);
-  } else {
-    if (hw) launch_pdl(k_fs1<S, C, M, true, false, kFs1Block>, grid, kFs1Block, st, q, tl, lc);
-    else launch_pdl(k_fs1<S, C, M, false, false, kFs1Block>, grid, kFs1Block, st, q, tl, lc);
-  }
+  auto go = [&](auto block, auto mb) {
+    constexpr int BLOCK = decltype(block)::value, MB = decltype(mb)::value;
+    if (hw) launch_pdl(k_fs1<S, C, M, true, false, BLOCK, MB>, grid, BLOCK, st, q, tl, lc);
+    else launch_pdl(k_fs1<S, C, M, false, false, BLOCK, MB>, grid, BLOCK, st, q, tl, lc);
+  };
+  using std::integral_constant;
+  if (tl.ntiles <= kTinyTiles) go(integral_constant<int, kFs1Small>{}, integral_constant<int, 1>{});
+  else if (tl.ntiles <= kSmallTiles) go(integral_constant<int, kFs1Small>{}, integral_constant<int, 2>{});
+  else go(integral_constant<int, kFs1Block>{}, integral_constant<int, 4>{});
 }
 
 template <class S, class C, class M>
@@ -129,54 +138,41 @@ void launch_apply_recon(const KParams& kp, cudaStream_t st, uint32_t odd) {
 // stream-collide drains (programmatic dependent launch); above, with an
 // ordinary launch (measured faster on the 8192x2048 dam break).  Returns the
 // number of kernels launched.
-template <class S, class C, class M, int TW, int CPT>
+template <class S, class C, class M, int TW, int CPT, int MB>
 void launch_fs234_form(const KParams& kp, cudaStream_t st, uint32_t odd, const TileList& tl, uint32_t grid,
                        uint32_t* nz, const NextLists& nl) {
   constexpr int threads = TW * kTY / CPT;
   const KParams q = as_even(kp, odd);
-  if (tl.ntiles <= kWideTiles) launch_pdl(k_fs234<S, C, M, false, TW, CPT>, grid, threads, st, q, tl, nz, nl);
-  else k_fs234<S, C, M, false, TW, CPT><<<grid, threads, 0, st>>>(q, tl, nz, nl);
+  if (tl.ntiles <= kWideTiles) launch_pdl(k_fs234<S, C, M, false, TW, CPT, MB>, grid, threads, st, q, tl, nz, nl);
+  else k_fs234<S, C, M, false, TW, CPT, MB><<<grid, threads, 0, st>>>(q, tl, nz, nl);
 }
 
 template <class S, class C, class M>
 int launch_fs234(const KParams& kp, cudaStream_t st, uint32_t odd, const TileList& tl, uint32_t grid, uint32_t* nz,
                  const NextLists& nl, int form) {
   switch (form) {
-    case FS_FORM_W32: launch_fs234_form<S, C, M, 32, 1>(kp, st, odd, tl, grid, nz, nl); break;
-    case FS_FORM_W64X1: launch_fs234_form<S, C, M, 64, 1>(kp, st, odd, tl, grid, nz, nl); break;
-    default: launch_fs234_form<S, C, M, 64, 2>(kp, st, odd, tl, grid, nz, nl); break;
+    case FS_FORM_W32: launch_fs234_form<S, C, M, 32, 1, 6>(kp, st, odd, tl, grid, nz, nl); break;
+    case FS_FORM_W64X1:
+      if (tl.ntiles <= kTinyTiles) launch_fs234_form<S, C, M, 64, 1, 2>(kp, st, odd, tl, grid, nz, nl);
+      else launch_fs234_form<S, C, M, 64, 1, 3>(kp, st, odd, tl, grid, nz, nl);
+      break;
+    default: launch_fs234_form<S, C, M, 64, 2, 4>(kp, st, odd, tl, grid, nz, nl); break;
   }
   return 1;
 }
 
-// Resident blocks per SM of FS_1 (which 0) or of the flag pass in the given
-// form (which 1).
-template <class S, class C, class M, int TW, int CPT>
-int fs234_blocks_per_sm() {
-  int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_fs234<S, C, M, false, TW, CPT>, TW * kTY / CPT, 0);
-  return n;
-}
-template <class S, class C, class M>
-int fs_blocks_per_sm(int which, int form) {
-  int n = 0;
-  if (which == 0 && form == 1)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_fs1<S, C, M, true, false, kFs1Small>, kFs1Small, 0);
-  else if (which == 0)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_fs1<S, C, M, true, false, kFs1Block>, kFs1Block, 0);
-  else if (form == FS_FORM_W32) n = fs234_blocks_per_sm<S, C, M, 32, 1>();
-  else if (form == FS_FORM_W64X1) n = fs234_blocks_per_sm<S, C, M, 64, 1>();
-  else n = fs234_blocks_per_sm<S, C, M, 64, 2>();
-  return n > 0 ? n : 1;
+// Resident blocks per SM: the launch bounds above.
+int fs1_blocks_per_sm(uint32_t ntiles) { return ntiles <= kTinyTiles ? 1 : ntiles <= kSmallTiles ? 2 : 4; }
+int fs234_blocks_per_sm(int form, uint32_t ntiles) {
+  return form == FS_FORM_W32 ? 6 : form == FS_FORM_W64X1 ? (ntiles <= kTinyTiles ? 2 : 3) : 4;
 }
 
 #define FLB_INSTANTIATE(S, C, M)                                                                                  \
   template void launch_fs1<S, C, M>(const KParams&, cudaStream_t, uint32_t, bool, const TileList&, uint32_t,       \
-                                    const ListClear&, bool);                                                     \
+                                    const ListClear&);                                                     \
   template void launch_apply_recon<S, C, M>(const KParams&, cudaStream_t, uint32_t);                             \
   template int launch_fs234<S, C, M>(const KParams&, cudaStream_t, uint32_t, const TileList&, uint32_t, uint32_t*,   \
-                                     const NextLists&, int);                                                     \
-  template int fs_blocks_per_sm<S, C, M>(int, int);
+                                     const NextLists&, int);
 FLB_FOR_EACH_VARIANT(FLB_INSTANTIATE)
 #undef FLB_INSTANTIATE
 

@@ -48,7 +48,7 @@ int sc_list_blocks_per_sm(bool vec, uint32_t ntiles);
 // FS_2..4 on listed super-tiles (appends the next step's lists)
 template <class S, class C, class M>
 void launch_fs1(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const TileList& tl, uint32_t grid,
-                const ListClear& lc, bool one_cell);
+                const ListClear& lc);
 template <class S, class C, class M>
 void launch_apply_recon(const KParams& kp, cudaStream_t st, uint32_t odd);
 template <class S, class C, class M>
@@ -57,10 +57,13 @@ int launch_fs234(const KParams& kp, cudaStream_t st, uint32_t odd, const TileLis
 // launch forms of the flag pass: tile width x cells per thread (threads per
 // block = width * 8 / cells per thread)
 enum FsForm { FS_FORM_W32 = 1, FS_FORM_W64X1 = 5, FS_FORM_W64X2 = 6 };
-// resident blocks per SM of FS_1 with `form` cells per thread (which 0) or of
-// the flag pass in `form` (which 1)
-template <class S, class C, class M>
-int fs_blocks_per_sm(int which, int form);
+// resident blocks per SM of FS_1 on a grid of ntiles super-tiles, and of the
+// flag pass in `form`
+int fs1_blocks_per_sm(uint32_t ntiles);
+int fs234_blocks_per_sm(int form, uint32_t ntiles);
+// up to this many super-tiles FS_1 and the flag pass take one cell per thread,
+// up to kTinyTiles FS_1 with all the registers (k_fs.cu)
+constexpr uint32_t kSmallTiles = 1024, kTinyTiles = 512;
 
 // the free-surface step as one persistent cooperative kernel (k_fsp.cu):
 // a.steps steps per launch, `grid` CTAs of 1024 threads all resident at once
