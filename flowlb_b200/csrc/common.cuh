@@ -195,6 +195,17 @@ __device__ __forceinline__ uint32_t tile_count(const TileList& tl) {
   return tl.all ? tl.ntiles : min(__ldcg(tl.count), tl.ntiles);
 }
 __device__ __forceinline__ uint32_t tile_at(const TileList& tl, uint32_t i) { return tl.all ? i : tl.list[i]; }
+// An entry of the FS_1 / stream-collide list: the super-tile, and kDeepTile when
+// it is deep: it lies inside the grid, and its cells and their neighbours are
+// all plain fluid (no wall next to them), so those passes read no flag or wall
+// mask there and wrap no neighbour.  The flag pass sets it from the window it
+// reads anyway.  Only on grids of more than kSmallTiles (kScSmallTiles)
+// super-tiles: the passes of a small grid run their code about once per block
+// and a second form of the cell costs them its instructions (1001x401 22.7 ->
+// 23.5 us per step, 300x120 13.3 -> 13.8).  Measured on a B200, us per step
+// without | with: 2048x512 FP32 23.4 | 22.6, FP64 28.0 | 26.5, 4001x1201 144 |
+// 140, 8192x2048 FP32 232 | 206, FP16S 227 | 197.
+constexpr uint32_t kDeepTile = 0x80000000u;
 
 // ---- L2 prefetch of a super-tile ------------------------------------------------
 // Bulk L2 prefetch (a hint with no reply) of `bytes` bytes from `p`, rounded
@@ -217,6 +228,7 @@ __device__ __forceinline__ void l2_prefetch_inward(const char* p, uint32_t bytes
 __device__ __forceinline__ void prefetch_super_tile(const KParams& p, uint32_t t, uint32_t nsx, uint32_t pop,
                                                    bool with_mass, uint32_t m) {
   const uint32_t k = threadIdx.x;
+  t &= ~kDeepTile;
   const uint32_t x0 = (t % nsx) * kSTW, y0 = (t / nsx) * kSTH;
   const uint32_t w = min(kSTW, p.nx - x0);
   int row = -1;

@@ -128,6 +128,37 @@ __device__ __forceinline__ void fs1_cell(const KParams& p, uint32_t x, uint32_t 
   fs1_cell<S, C, M, HW, ODD>(p, x, y, flag, nbm);
 }
 
+// A cell of a deep super-tile: fluid, as all its neighbours, none of them
+// across the grid's edge or a wall.
+template <class S, class C, class M, bool ODD>
+__device__ __forceinline__ void fs1_deep_cell(const KParams& p, uint32_t idx) {
+  const uint32_t nx = p.nx;
+  const uint32_t nb[9] = {idx,          idx + 1u,      idx - 1u,      idx + nx,      idx - nx,
+                          idx + nx + 1u, idx - nx - 1u, idx - nx + 1u, idx + nx - 1u};
+  C in[9], out[9];
+  const float inv = p.f16_inv;
+#pragma unroll
+  for (int i = 1; i < 9; i += 2) {
+    in[i] = Codec<S, C>::ld(slotp<S>(p, slot_a<ODD>(i)), idx, i, inv);
+    in[i + 1] = Codec<S, C>::ld(slotp<S>(p, slot_b<ODD>(i)), nb[i], i + 1, inv);
+  }
+  load_out<S, C, ODD>(p, idx, nb, out);
+  M* Ms = static_cast<M*>(p.mass);
+  const M* Ex = static_cast<const M*>(p.excess);
+  M m = Ms[idx];
+  M exn[9];
+#pragma unroll
+  for (int i = 1; i < 9; i++) exn[i] = Ex[nb[i]];
+#pragma unroll
+  for (int i = 1; i < 9; i++) m += exn[i];
+#pragma unroll
+  for (int i = 1; i < 9; i += 2) {
+    m += in[i + 1] - out[i];
+    m += in[i] - out[i + 1];
+  }
+  Ms[idx] = m;
+}
+
 // ---- FS_2 + FS_3 + FS_4 fused: lbmKernel2D.cu:124-303 ----------------------
 // The three reference passes are flag stencils of radius one, chained; a tile
 // of kTX x 8 cells stages the flags of its 3-cell halo in shared memory and
@@ -428,6 +459,18 @@ __device__ __forceinline__ bool fs234_cell(const KParams& p, const FlagMasks<TW>
   return live;
 }
 
+// The same for a cell of a tile whose whole window is plain fluid: its flag
+// stays, it is full, and it hands what it has too much to its eight neighbours.
+template <class C, class M>
+__device__ __forceinline__ void fs234_deep_cell(const KParams& p, uint32_t idx, const Fs4Own<C, M>& own) {
+  const bool trust = p.trust_prev != 0;
+  if (!trust || own.old != own.f0) p.flags_out[idx] = own.f0;
+  const M ex = own.m - own.rho;
+  static_cast<M*>(p.mass)[idx] = M(own.rho) + M(0);
+  static_cast<M*>(p.excess)[idx] = div_count(ex, 8);
+  if (!trust) static_cast<M*>(p.phi)[idx] = 1.0f;
+}
+
 // The general stencil stages of the flag pass on a tile (every thread of the
 // block calls it): the masks of the flags after stream-collide (from the flag
 // bytes fv each warp loaded), FS_2 and FS_3 as dilations and word logic, and
@@ -538,10 +581,11 @@ __device__ __forceinline__ void load_window(const KParams& p, int tx, int ty, in
 // block, CPT cells per thread (rows ly and ly + 8/CPT, ...); every thread of
 // the block must call it.  Returns the activity bits (activity, above) of
 // this thread's cells that are fluid or interface after the pass, with the
-// tile at column xoff of a super-tile of wact x hact cells.
-template <class S, class C, class M, bool ODD, int TW, int CPT>
+// tile at column xoff of a super-tile of wact x hact cells.  deep: the window
+// is all plain fluid.
+template <class S, class C, class M, bool ODD, int TW, int CPT, bool DEEP>
 __device__ __forceinline__ uint32_t fs234_tile(const KParams& p, int tx, int ty, int tid, FlagMasks<TW>& sm,
-                                               int xoff, int wact, int hact) {
+                                               int xoff, int wact, int hact, bool& deep) {
   constexpr int kTX = TW, kW = FlagMasks<TW>::kW, kR = FlagMasks<TW>::kR;
   constexpr int kThreads = TW * kTY / CPT, kWarps = kThreads / 32, kRowStep = kTY / CPT;
   static_assert(kTY % CPT == 0 && kThreads >= (kR - 2) * kW, "flag pass: block too small for the stencil stages");
@@ -566,6 +610,26 @@ __device__ __forceinline__ uint32_t fs234_tile(const KParams& p, int tx, int ty,
   for (int k = 0; k < CPT; k++) {
     const int gy = ty * kTY + ly0 + k * kRowStep;
     if (gx < nx && gy < ny) fs4_own_excess<C, M>(p, (uint32_t)gx + (uint32_t)gy * (uint32_t)nx, own[k]);
+  }
+  // most listed tiles of a large grid are deep fluid: every byte of the window
+  // is plain fluid
+  if constexpr (DEEP) {
+    bool nd = false;
+#pragma unroll
+    for (int k = 0; k < kIters; k++) nd |= (tid >> 5) + k * kWarps < kRW && fv[k] != kFluid;
+    deep = __syncthreads_or(nd) == 0;
+    if (deep) {
+      uint32_t act = 0;
+#pragma unroll
+      for (int k = 0; k < CPT; k++) {
+        const int ly = ly0 + k * kRowStep, gy = ty * kTY + ly;
+        if (gx < nx && gy < ny) {
+          fs234_deep_cell<C, M>(p, (uint32_t)gx + (uint32_t)gy * (uint32_t)nx, own[k]);
+          act |= activity(xoff + lx, ly, wact, hact);
+        }
+      }
+      return act;
+    }
   }
   bool nq = false;
 #pragma unroll
@@ -593,9 +657,9 @@ __device__ __forceinline__ uint32_t fs234_tile(const KParams& p, int tx, int ty,
 // bit 0: the flag-pass list), and the neighbour in the direction of every set
 // edge bit of m (the flag-pass list).  A super-tile is added to the flag-pass
 // list once (the first to set its mark adds it).  The lengths never pass the
-// super-tile count, whatever the state of the marks.
+// super-tile count, whatever the state of the marks.  deep: see kDeepTile.
 __device__ __forceinline__ void append_next(const NextLists& nl, uint32_t t, uint32_t m, uint32_t old,
-                                            uint32_t lane) {
+                                            bool deep, uint32_t lane) {
   constexpr uint32_t kNone = 0xffffffffu;
   const uint32_t T = nl.nsx * nl.nsy;
   uint32_t cand = kNone;
@@ -627,14 +691,14 @@ __device__ __forceinline__ void append_next(const NextLists& nl, uint32_t t, uin
     const uint32_t k = base_fs + __popc(bfs & ((1u << lane) - 1u));
     if (k < T) nl.list_fs[k] = cand;
   }
-  if (add_sc && base_sc < T) nl.list_sc[base_sc] = t;
+  if (add_sc && base_sc < T) nl.list_sc[base_sc] = deep ? t | kDeepTile : t;
 }
 
 // The flag pass over one super-tile t (its kSTW / TW tiles in turn) with the
 // TW*kTY/CPT threads of the block; every thread of the block must call it.
 // Records the super-tile's activity word in nz[t] (whose previous value, the
 // word of the last step, it reads first) and appends to the next step's lists.  wact_sm: one word per warp of the block.
-template <class S, class C, class M, bool ODD, int TW, int CPT = 1>
+template <class S, class C, class M, bool ODD, int TW, int CPT = 1, bool DEEP = false>
 __device__ __forceinline__ void fs234_super_tile(const KParams& p, uint32_t t, uint32_t nsx, uint32_t* nz,
                                                  const NextLists& nl, FlagMasks<TW>& sm, uint32_t* wact_sm) {
   constexpr int kTX = TW, kWarps = TW * kTY / CPT / 32;
@@ -642,6 +706,8 @@ __device__ __forceinline__ void fs234_super_tile(const KParams& p, uint32_t t, u
   const int sx = (int)(t % nsx), sy = (int)(t / nsx);
   const int wact = min((int)kSTW, (int)p.nx - sx * (int)kSTW), hact = min((int)kSTH, (int)p.ny - sy * (int)kSTH);
   uint32_t act = 0;
+  // deep (kDeepTile): inside the grid and every tile of it deep
+  bool all_deep = DEEP && sx > 0 && sy > 0 && (uint32_t)(sx + 1) * kSTW < p.nx && (uint32_t)(sy + 1) * kSTH < p.ny;
   // the word of the last step, read now so that its latency overlaps the
   // tile (only this block writes nz[t] during the pass, at the end)
   const uint32_t word = tid < 32 ? __ldcg(nz + t) : 0u;
@@ -651,7 +717,11 @@ __device__ __forceinline__ void fs234_super_tile(const KParams& p, uint32_t t, u
 #pragma unroll 1
   for (int j = 0; j < (int)(kSTW / kTX); j++) {
     const int tx = sx * (int)(kSTW / kTX) + j;
-    if (tx * kTX < (int)p.nx) act |= fs234_tile<S, C, M, ODD, TW, CPT>(p, tx, sy, tid, sm, j * kTX, wact, hact);
+    if (tx * kTX < (int)p.nx) {
+      bool deep = false;
+      act |= fs234_tile<S, C, M, ODD, TW, CPT, DEEP>(p, tx, sy, tid, sm, j * kTX, wact, hact, deep);
+      all_deep &= deep;
+    }
   }
   act = __reduce_or_sync(0xffffffffu, act);
   if ((tid & 31) == 0) wact_sm[tid >> 5] = act;
@@ -659,7 +729,7 @@ __device__ __forceinline__ void fs234_super_tile(const KParams& p, uint32_t t, u
   if (tid < 32) {
     const uint32_t m = __reduce_or_sync(0xffffffffu, tid < kWarps ? wact_sm[tid] : 0u);
     if (tid == 0) nz[t] = m;
-    append_next(nl, t, m, word, (uint32_t)tid);
+    append_next(nl, t, m, word, all_deep, (uint32_t)tid);
   }
 }
 

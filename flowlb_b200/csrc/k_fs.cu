@@ -26,7 +26,7 @@ constexpr int kFs1Block = 256;   // two cells per thread (x and x + 32 of a row)
 constexpr int kFs1Small = 512;   // one cell per thread, two blocks per SM, or one
 // lc: the next step's list lengths and marks, cleared here for this step's
 // flag pass.
-template <class S, class C, class M, bool HW, bool ODD, int BLOCK, int MB>
+template <class S, class C, class M, bool HW, bool ODD, int BLOCK, int MB, bool DEEP>
 __global__ void __launch_bounds__(BLOCK, MB) k_fs1(const __grid_constant__ KParams p,
                                                                        const TileList tl, const ListClear lc) {
   pdl_wait();
@@ -46,9 +46,16 @@ __global__ void __launch_bounds__(BLOCK, MB) k_fs1(const __grid_constant__ KPara
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x, t = i < n ? tile_at(tl, i) : 0u) {
     // the block's next super-tile into L2 while this one is worked on
     if (i + gridDim.x < n) prefetch_super_tile(p, tile_at(tl, i + gridDim.x), tl.nsx, sizeof(S), true, sizeof(M));
+    const bool deep = DEEP && (t & kDeepTile);
+    t &= ~kDeepTile;
     const uint32_t y = (t / tl.nsx) * kSTH + row;
     if (y >= p.ny) continue;
     const uint32_t xa = (t % tl.nsx) * kSTW + chunk * 32u + lane, xc = xa + 32u * kCpr;
+    if (deep) {
+#pragma unroll
+      for (uint32_t k = 0; k < kCells; k++) fs1_deep_cell<S, C, M, ODD>(p, xa + 32u * kCpr * k + y * nx);
+      continue;
+    }
     // the cells' flags and wall masks first: one round trip for both
     uint8_t fa = kGas, fc = kGas;
     uint32_t ma = 0, mc = 0;
@@ -108,7 +115,7 @@ __global__ void __launch_bounds__(TW* kTY / CPT, MB)
   pdl_wait();
   pdl_trigger();
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x)
-    fs234_super_tile<S, C, M, ODD, TW, CPT>(p, tile_at(tl, i), tl.nsx, nz, nl, sm, wact_sm);
+    fs234_super_tile<S, C, M, ODD, TW, CPT, (CPT > 1)>(p, tile_at(tl, i), tl.nsx, nz, nl, sm, wact_sm);
 }
 
 // ---- launchers -------------------------------------------------------------------
@@ -118,8 +125,9 @@ void launch_fs1(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const
   const KParams q = as_even(kp, odd);
   auto go = [&](auto block, auto mb) {
     constexpr int BLOCK = decltype(block)::value, MB = decltype(mb)::value;
-    if (hw) launch_pdl(k_fs1<S, C, M, true, false, BLOCK, MB>, grid, BLOCK, st, q, tl, lc);
-    else launch_pdl(k_fs1<S, C, M, false, false, BLOCK, MB>, grid, BLOCK, st, q, tl, lc);
+    constexpr bool DEEP = BLOCK == kFs1Block;
+    if (hw) launch_pdl(k_fs1<S, C, M, true, false, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl, lc);
+    else launch_pdl(k_fs1<S, C, M, false, false, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl, lc);
   };
   using std::integral_constant;
   if (tl.ntiles <= kTinyTiles) go(integral_constant<int, kFs1Small>{}, integral_constant<int, 1>{});

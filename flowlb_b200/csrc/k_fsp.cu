@@ -101,14 +101,14 @@ __device__ __forceinline__ bool fsp_step(const KParams& p, const uint32_t odd, c
   clear_next_lists(ListClear{a.lcount + 2 * (odd ^ 1u), a.lbits + (odd ^ 1u) * a.nwords, a.nwords});
   // FS_1: mass exchange and gas reconstruction
   for (uint32_t i = blockIdx.x; i < nsc; i += G) {
-    const uint32_t t = __ldcg(lsc + i);
+    const uint32_t t = __ldcg(lsc + i) & ~kDeepTile;
     const uint32_t y = (t / a.nsx) * kSTH + row, x = (t % a.nsx) * kSTW + xo;
     if (y < p.ny && x < p.nx) fs1_cell<S, C, M, HW, false>(p, x, y);
   }
   if (!next_barrier(a, nbar, ok)) return false;
   // stream-collide
   for (uint32_t i = blockIdx.x; i < nsc; i += G) {
-    const uint32_t t = __ldcg(lsc + i);
+    const uint32_t t = __ldcg(lsc + i) & ~kDeepTile;
     const uint32_t y = (t / a.nsx) * kSTH + row, x = (t % a.nsx) * kSTW + xo;
     if (y < p.ny && x < p.nx) sc_cell<S, C, M, true, HW, true, false, FU>(p, x, y);
   }

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kBlock, FLB_SC_MIN_BLOCKS) k_sc_scalar(const _
 // where FP32 with the fused arithmetic (few spills at 32 registers) is bound by
 // memory (more than kScLargeTiles super-tiles), 256 x 4 elsewhere.
 constexpr uint32_t kScSmallTiles = 1024, kScLargeTiles = 8192;
-template <class S, class C, class M, bool HW, bool ODD, bool FU, int BLOCK, int MB>
+template <class S, class C, class M, bool HW, bool ODD, bool FU, int BLOCK, int MB, bool DEEP>
 __global__ void __launch_bounds__(BLOCK, MB) k_sc_list(const __grid_constant__ KParams p,
                                                                            const TileList tl) {
   // the list was built two kernels back (FS_1 waited for it), so it is read
@@ -75,10 +75,15 @@ __global__ void __launch_bounds__(BLOCK, MB) k_sc_list(const __grid_constant__ K
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t row = warp % kSTH, chunk = warp / kSTH, cpr = (blockDim.x >> 5) / kSTH;
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-    const uint32_t t = tile_at(tl, i);
+    const uint32_t e = tile_at(tl, i), t = e & ~kDeepTile;
     const uint32_t y = (t / tl.nsx) * kSTH + row;
     if (y >= p.ny) continue;
     const uint32_t xb = (t % tl.nsx) * kSTW + lane;
+    if (DEEP && (e & kDeepTile)) {
+#pragma unroll 1
+      for (uint32_t j = chunk * 32u; j < kSTW; j += 32u * cpr) sc_deep_cell<S, C, M, ODD, FU>(p, xb + j, y);
+      continue;
+    }
 #pragma unroll 1
     for (uint32_t j = chunk * 32u; j < kSTW; j += 32u * cpr)
       if (xb + j < p.nx) sc_cell<S, C, M, true, HW, true, ODD, FU>(p, xb + j, y);
@@ -320,7 +325,7 @@ __global__ void __launch_bounds__(list_vec_block<S>(), 1024 / list_vec_block<S>(
   pdl_trigger();
   const uint32_t lane = threadIdx.x % LPR, row = threadIdx.x / LPR;
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-    const uint32_t t = tile_at(tl, i);
+    const uint32_t t = tile_at(tl, i) & ~kDeepTile;
     const uint32_t y = (t / tl.nsx) * kSTH + row;
     const uint32_t x0 = y < p.ny ? (t % tl.nsx) * kSTW + lane * V : p.nx;
     sc_vec_cells<S, C, M, true, HW, true, ODD, FU, LPR>(p, x0, y < p.ny ? y : 0u, lane);
@@ -644,8 +649,9 @@ static void launch_sc_list_f(const KParams& kp, cudaStream_t st, uint32_t odd, b
   }
   auto go = [&](auto block, auto mb) {
     constexpr int BLOCK = decltype(block)::value, MB = decltype(mb)::value;
-    if (hw) launch_pdl(k_sc_list<S, C, M, true, false, FU, BLOCK, MB>, grid, BLOCK, st, q, tl);
-    else launch_pdl(k_sc_list<S, C, M, false, false, FU, BLOCK, MB>, grid, BLOCK, st, q, tl);
+    constexpr bool DEEP = MB == 4;
+    if (hw) launch_pdl(k_sc_list<S, C, M, true, false, FU, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl);
+    else launch_pdl(k_sc_list<S, C, M, false, false, FU, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl);
   };
   using std::integral_constant;
   if (tl.ntiles <= kScSmallTiles) go(integral_constant<int, 512>{}, integral_constant<int, 2>{});
