@@ -140,6 +140,7 @@ struct NextLists {
   uint32_t* counts;  // [2]: lengths of list_sc and list_fs
   uint32_t* bits;    // (ntiles + 31) / 32 words
   uint32_t nsx, nsy;
+  uint32_t thin;     // the last super-tile column (1) or row (2) is narrower than the flag pass's reach
 };
 struct ListClear {
   uint32_t* counts;  // [2]
@@ -180,7 +181,7 @@ struct FspArgs {
   uint32_t nwords;
   uint32_t* nz;
   uint32_t nsx, nsy;
-  int fs_all;            // the flag pass visits every super-tile (thin last super-tiles)
+  uint32_t thin;         // NextLists::thin
   uint32_t* bar;         // grid barrier arrivals, zeroed before each launch
   uint32_t* err;         // set when a barrier wait gave up
   uint32_t steps;        // even: the run starts at an even t with flag buffer 0 current

@@ -81,7 +81,7 @@ struct flb_engine {
   // the previous step visited every super-tile: this step's flag pass must
   // too (the activity words of two steps back are unknown)
   bool fs_all_next = false;
-  bool thin_tiles = false;        // a last super-tile column or row narrower than the flag pass's reach
+  uint32_t thin = 0;              // NextLists::thin
   uint32_t grid_sc = 0, grid_fs1 = 0, grid_fs234 = 0;
   // persistent free-surface step (k_fsp.cu): requested mode, resolved path,
   // resident grid, barrier count and error word
@@ -262,13 +262,11 @@ struct FsLists {
   bool all;
 };
 
-// A live cell can reach past a super-tile narrower than 3 cells into the one
-// beyond it; such grids visit every super-tile in the flag pass.
 FsLists fs_lists(flb_engine* h, uint64_t t) {
   const int lp = (int)(t & 1u);
   FsLists L;
   L.all = !h->lists_valid;
-  const bool fs_all = L.all || h->fs_all_next || h->thin_tiles;
+  const bool fs_all = L.all || h->fs_all_next;
   L.sc = TileList{h->d_list[lp][0], h->d_lcount + 2 * lp, h->ntiles, h->nsx, L.all ? 1 : 0};
   L.fs = TileList{h->d_list[lp][1], h->d_lcount + 2 * lp + 1, h->ntiles, h->nsx, fs_all ? 1 : 0};
   L.next_count = h->d_lcount + 2 * (lp ^ 1);
@@ -280,7 +278,7 @@ FsLists fs_lists(flb_engine* h, uint64_t t) {
 NextLists next_lists(flb_engine* h, uint64_t t) {
   const int np = (int)((t + 1) & 1u);
   return NextLists{h->d_list[np][0], h->d_list[np][1], h->d_lcount + 2 * np, h->d_lbits + (size_t)np * h->nwords,
-                   h->nsx, h->nsy};
+                   h->nsx, h->nsy, h->thin};
 }
 ListClear list_clear(flb_engine* h, uint64_t t) {
   const NextLists nl = next_lists(h, t);
@@ -367,7 +365,7 @@ flb_status issue_persist(flb_engine* h, int pairs, uint64_t* trace = nullptr) {
   a.nz = h->d_nz;
   a.nsx = h->nsx;
   a.nsy = h->nsy;
-  a.fs_all = h->thin_tiles ? 1 : 0;
+  a.thin = h->thin;
   a.bar = h->d_bar;
   a.err = h->d_perr;
   a.steps = 2u * (uint32_t)pairs;
@@ -880,7 +878,7 @@ FLB_API flb_status flb_create(const flb_case_desc* desc, flb_handle* out) {
   const uint64_t blocks = (N + kBlock - 1) / kBlock;
   h->nsx = (h->nx + kSTW - 1) / kSTW;
   h->nsy = (h->ny + kSTH - 1) / kSTH;
-  h->thin_tiles = (h->nx % kSTW != 0 && h->nx % kSTW < 3) || (h->ny % kSTH != 0 && h->ny % kSTH < 3);
+  h->thin = (h->nx % kSTW != 0 && h->nx % kSTW < 3 ? 1u : 0u) | (h->ny % kSTH != 0 && h->ny % kSTH < 3 ? 2u : 0u);
   h->ntiles = h->nsx * h->nsy;
   h->nwords = (h->ntiles + 31u) / 32u;
   const uint64_t tiles = h->ntiles;

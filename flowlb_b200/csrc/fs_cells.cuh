@@ -651,6 +651,27 @@ __device__ __forceinline__ uint32_t fs234_tile(const KParams& p, int tx, int ty,
   return act;
 }
 
+// A live cell of super-tile t reaches past a last super-tile column or row of
+// one or two cells into the super-tile beyond it.  The j-th (0..15) of the
+// super-tiles two away in x or y, if it is one of those and t's word m says that
+// live cells face it, else kNoTile.  (Visiting every super-tile on such grids
+// instead: 4001x1201 140 us per step against 67.7, 1001x401 22.7 against 18.9.)  THIN
+// tells grids that have one: elsewhere the code costs the 64-register flag pass
+// 5% (2048x512 FP64 26.4 -> 27.6 us per step).
+constexpr uint32_t kNoTile = 0xffffffffu;
+__device__ __forceinline__ uint32_t beyond_thin(const NextLists& nl, uint32_t t, uint32_t m, int j) {
+  const int ox = j < 5 ? 2 : j < 10 ? -2 : j < 13 ? j - 11 : j - 14;
+  const int oy = j < 5 ? j - 2 : j < 10 ? j - 7 : j < 13 ? 2 : -2;
+  const int nsx = (int)nl.nsx, nsy = (int)nl.nsy, sx = (int)(t % nl.nsx), sy = (int)(t / nl.nsx);
+  if (!((m >> edge_bit(ox > 0 ? 1 : ox < 0 ? -1 : 0, oy > 0 ? 1 : oy < 0 ? -1 : 0)) & 1u)) return kNoTile;
+  // two steps lead over the last column / row only from the one before it or,
+  // across the periodic edge, from the first
+  const bool x2 = (nl.thin & 1u) && nsx > 1 && (ox > 0 ? sx + 2 == nsx : sx == 0);
+  const bool y2 = (nl.thin & 2u) && nsy > 1 && (oy > 0 ? sy + 2 == nsy : sy == 0);
+  if (((ox == 2 || ox == -2) && !x2) || ((oy == 2 || oy == -2) && !y2)) return kNoTile;
+  return (uint32_t)wrapi(sx + ox, nsx) + (uint32_t)wrapi(sy + oy, nsy) * nl.nsx;
+}
+
 // Appends super-tile t to the next step's lists (NextLists), with warp 0 of
 // the block (every lane calls it): t itself when it holds fluid or interface
 // cells now (m bit 0: both lists) or held some after the previous step (old
@@ -658,11 +679,11 @@ __device__ __forceinline__ uint32_t fs234_tile(const KParams& p, int tx, int ty,
 // edge bit of m (the flag-pass list).  A super-tile is added to the flag-pass
 // list once (the first to set its mark adds it).  The lengths never pass the
 // super-tile count, whatever the state of the marks.  deep: see kDeepTile.
+template <bool THIN>
 __device__ __forceinline__ void append_next(const NextLists& nl, uint32_t t, uint32_t m, uint32_t old,
                                             bool deep, uint32_t lane) {
-  constexpr uint32_t kNone = 0xffffffffu;
   const uint32_t T = nl.nsx * nl.nsy;
-  uint32_t cand = kNone;
+  uint32_t cand = kNoTile;
   if (lane == 0) {
     if ((m | old) & 1u) cand = t;
   } else if (lane <= 8u && ((m >> lane) & 1u)) {
@@ -673,6 +694,8 @@ __device__ __forceinline__ void append_next(const NextLists& nl, uint32_t t, uin
     const uint32_t xx = dx > 0 ? (sx + 1u == nl.nsx ? 0u : sx + 1u) : dx < 0 ? (sx == 0u ? nl.nsx - 1u : sx - 1u) : sx;
     const uint32_t yy = dy > 0 ? (sy + 1u == nl.nsy ? 0u : sy + 1u) : dy < 0 ? (sy == 0u ? nl.nsy - 1u : sy - 1u) : sy;
     cand = xx + yy * nl.nsx;
+  } else if (THIN && lane >= 9u && lane < 25u) {
+    cand = beyond_thin(nl, t, m, (int)lane - 9);
   }
   // the stream-collide slot is taken beside the marks (independent atomics,
   // so their round trips overlap)
@@ -680,7 +703,7 @@ __device__ __forceinline__ void append_next(const NextLists& nl, uint32_t t, uin
   uint32_t base_fs = 0, base_sc = 0;
   if (add_sc) base_sc = atomicAdd(nl.counts, 1u);
   bool add_fs = false;
-  if (cand != kNone) {
+  if (cand != kNoTile) {
     const uint32_t bit = 1u << (cand & 31u);
     add_fs = (atomicOr(nl.bits + (cand >> 5), bit) & bit) == 0u;
   }
@@ -698,7 +721,7 @@ __device__ __forceinline__ void append_next(const NextLists& nl, uint32_t t, uin
 // TW*kTY/CPT threads of the block; every thread of the block must call it.
 // Records the super-tile's activity word in nz[t] (whose previous value, the
 // word of the last step, it reads first) and appends to the next step's lists.  wact_sm: one word per warp of the block.
-template <class S, class C, class M, bool ODD, int TW, int CPT = 1, bool DEEP = false>
+template <class S, class C, class M, bool ODD, int TW, int CPT, bool DEEP, bool THIN>
 __device__ __forceinline__ void fs234_super_tile(const KParams& p, uint32_t t, uint32_t nsx, uint32_t* nz,
                                                  const NextLists& nl, FlagMasks<TW>& sm, uint32_t* wact_sm) {
   constexpr int kTX = TW, kWarps = TW * kTY / CPT / 32;
@@ -729,7 +752,7 @@ __device__ __forceinline__ void fs234_super_tile(const KParams& p, uint32_t t, u
   if (tid < 32) {
     const uint32_t m = __reduce_or_sync(0xffffffffu, tid < kWarps ? wact_sm[tid] : 0u);
     if (tid == 0) nz[t] = m;
-    append_next(nl, t, m, word, all_deep, (uint32_t)tid);
+    append_next<THIN>(nl, t, m, word, all_deep, (uint32_t)tid);
   }
 }
 

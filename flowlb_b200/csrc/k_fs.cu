@@ -104,7 +104,7 @@ __global__ void k_apply_recon(const __grid_constant__ KParams p, uint32_t odd) {
 // registers: 300x120 14.4 against 13.4 us per step with FS_1's form), three
 // above (1001x401 22.8 against 23.4); with two cells four (five spill at 48:
 // 2048x512 25.1 against 24.2, 4001x1201 159 against 148).
-template <class S, class C, class M, bool ODD, int TW, int CPT, int MB>
+template <class S, class C, class M, bool ODD, int TW, int CPT, int MB, bool THIN>
 __global__ void __launch_bounds__(TW* kTY / CPT, MB)
     k_fs234(const __grid_constant__ KParams p, const TileList tl, uint32_t* __restrict__ nz, const NextLists nl) {
   __shared__ FlagMasks<TW> sm;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(TW* kTY / CPT, MB)
   pdl_wait();
   pdl_trigger();
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x)
-    fs234_super_tile<S, C, M, ODD, TW, CPT, (CPT > 1)>(p, tile_at(tl, i), tl.nsx, nz, nl, sm, wact_sm);
+    fs234_super_tile<S, C, M, ODD, TW, CPT, (CPT > 1), THIN>(p, tile_at(tl, i), tl.nsx, nz, nl, sm, wact_sm);
 }
 
 // ---- launchers -------------------------------------------------------------------
@@ -151,8 +151,13 @@ void launch_fs234_form(const KParams& kp, cudaStream_t st, uint32_t odd, const T
                        uint32_t* nz, const NextLists& nl) {
   constexpr int threads = TW * kTY / CPT;
   const KParams q = as_even(kp, odd);
-  if (tl.ntiles <= kWideTiles) launch_pdl(k_fs234<S, C, M, false, TW, CPT, MB>, grid, threads, st, q, tl, nz, nl);
-  else k_fs234<S, C, M, false, TW, CPT, MB><<<grid, threads, 0, st>>>(q, tl, nz, nl);
+  auto go = [&](auto thin) {
+    constexpr bool THIN = decltype(thin)::value;
+    if (tl.ntiles <= kWideTiles) launch_pdl(k_fs234<S, C, M, false, TW, CPT, MB, THIN>, grid, threads, st, q, tl, nz, nl);
+    else k_fs234<S, C, M, false, TW, CPT, MB, THIN><<<grid, threads, 0, st>>>(q, tl, nz, nl);
+  };
+  if (nl.thin) go(std::true_type{});
+  else go(std::false_type{});
 }
 
 template <class S, class C, class M>

@@ -95,7 +95,7 @@ __device__ __forceinline__ bool fsp_step(const KParams& p, const uint32_t odd, c
   // lengths of this step's lists (built by the previous step)
   const uint32_t T = a.nsx * a.nsy;
   const uint32_t nsc = min(__ldcg(a.lcount + 2 * odd), T);
-  const uint32_t nfs = a.fs_all ? T : min(__ldcg(a.lcount + 2 * odd + 1), T);
+  const uint32_t nfs = min(__ldcg(a.lcount + 2 * odd + 1), T);
   // the next step's list lengths and marks, which this step's flag pass
   // appends to (the previous step's passes have finished reading them)
   clear_next_lists(ListClear{a.lcount + 2 * (odd ^ 1u), a.lbits + (odd ^ 1u) * a.nwords, a.nwords});
@@ -116,9 +116,9 @@ __device__ __forceinline__ bool fsp_step(const KParams& p, const uint32_t odd, c
   // FS_2..4: flag stencil, mass / excess / fill level, activity words and the
   // next step's lists
   const NextLists nl{a.list[odd ^ 1u][0], a.list[odd ^ 1u][1], a.lcount + 2 * (odd ^ 1u), a.lbits + (odd ^ 1u) * a.nwords,
-                     a.nsx, a.nsy};
+                     a.nsx, a.nsy, a.thin};
   for (uint32_t i = blockIdx.x; i < nfs; i += G)
-    fs234_super_tile<S, C, M, false, 64>(p, a.fs_all ? i : __ldcg(lfs + i), a.nsx, a.nz, nl, sm, wact_sm);
+    fs234_super_tile<S, C, M, false, 64, 1, false, true>(p, __ldcg(lfs + i), a.nsx, a.nz, nl, sm, wact_sm);
   return next_barrier(a, nbar, ok);
 }
 

@@ -1,0 +1,67 @@
+"""Free-surface super-tile lists against the CPU oracle on grids whose last
+super-tile column or row is one or two cells wide, and on grids with super-tiles
+of plain fluid, with liquid that crosses the periodic edges: every field equal."""
+import numpy as np
+import pytest
+
+from conftest import exact_equal, first_mismatch
+from flowlb_b200 import cases
+from flowlb_b200 import engine as E
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("f", "rho", "u", "flags", "mass", "excess", "phi")
+
+
+def blobs(nx, ny, walls):
+    """Liquid around the periodic corner and in the middle, gas elsewhere."""
+    y, x = np.mgrid[0:ny, 0:nx]
+    dx, dy = np.minimum(x, nx - x) / nx, np.minimum(y, ny - y) / ny
+    flags = np.full((ny, nx), cases.GAS, np.uint8)
+    flags[(dx < 0.3) & (dy < 0.35)] = cases.FLUID
+    flags[(np.abs(x - 0.55 * nx) < 0.08 * nx) & (np.abs(y - 0.6 * ny) < 0.2 * ny)] = cases.FLUID
+    if walls:
+        flags[0, :] = cases.WALL
+        flags[ny // 3:ny // 3 + 2, nx // 4:nx // 4 + 3] = cases.WALL
+    return flags
+
+
+def oracle_fields(o, prec):
+    f = o.f64()
+    return dict(f=f if prec == 64 else f.astype(np.float32), rho=o.rho, u=o.u, flags=o.flags, mass=o.mass,
+                excess=o.excess, phi=o.phi)
+
+
+# thin in x, in y, in both, in neither; up to 512, 1024 and more super-tiles
+@pytest.mark.parametrize("nx,ny", [(65, 10), (130, 21), (66, 9), (3, 17), (96, 3), (321, 402), (1601, 265),
+                                   (2113, 266), (2176, 520)], ids=lambda v: str(v))
+@pytest.mark.parametrize("prec,walls,mode", [(32, False, E.STEP_KERNELS), (64, True, E.STEP_KERNELS),
+                                             (16, True, E.STEP_KERNELS), (32, True, E.STEP_PERSISTENT)],
+                         ids=["f32", "f64-walls", "f16s-walls", "f32-walls-persistent"])
+def test_lists_match_oracle(nx, ny, prec, walls, mode):
+    flags = blobs(nx, ny, walls)
+    kw = dict(tau=0.56, fx=3e-4, fy=-2e-4, u_max=0.25)
+    s = E.Solver(flags, free_surface=True, precision=prec, mass_precision=64, bounce_back=E.BB_HALFWAY,
+                 fs_mode=E.FS_CONSERVATIVE, arithmetic=E.ARITH_FUSED, **kw)
+    s.set_step_mode(mode)
+    variant = {32: O.F32, 64: O.F64, 16: O.F16S}[prec]
+    o = O.Oracle(flags, O.OracleConfig(variant=variant, free_surface=True, bb=O.BB_HALFWAY,
+                                       fs_mode=O.FS_CONSERVATIVE, arithmetic=O.ARITH_FUSED, **kw))
+    for n in (1, 2, 5, 60):
+        s.step(n)
+        o.step(n)
+        want = oracle_fields(o, prec)
+        for name in FIELDS:
+            a = getattr(s, name)
+            assert exact_equal(a, want[name]), f"t={o.t} {name}: {first_mismatch(a, want[name])}"
+    if mode == E.STEP_KERNELS:
+        s.set_step_mode(E.STEP_PERSISTENT)  # the other form takes over the lists
+        s.step(34)
+        o.step(34)
+        want = oracle_fields(o, prec)
+        for name in FIELDS:
+            a = getattr(s, name)
+            assert exact_equal(a, want[name]), f"t={o.t} {name}: {first_mismatch(a, want[name])}"
+    s.close()
+    o.close()
