@@ -494,6 +494,7 @@ struct flb_batch_s {
   std::vector<flb_case_desc> descs;  // the cases (flags point into hgeo)
   std::vector<uint8_t> hgeo;         // host copy of every case's geometry flags
   std::vector<flb_handle> handles;
+  char* d_second = nullptr;  // their second population buffers
   std::vector<uint32_t> stream_of;   // the pool stream of each case
   std::vector<uint32_t> sorder;      // the cases longest first
   std::vector<cudaStream_t> pool;
@@ -551,6 +552,7 @@ void bfree(flb_batch b) {
   for (flb_handle h : b->handles)
     if (h) flb_destroy(h);
   b->handles.clear();
+  if (b->d_second) cudaFree(b->d_second);
   for (cudaStream_t st : b->pool) cudaStreamDestroy(st);
   for (cudaEvent_t ev : b->pool_ev) cudaEventDestroy(ev);
   b->pool.clear();
@@ -801,6 +803,8 @@ void streams_free(flb_batch b) {
   for (flb_handle h : b->handles)
     if (h) flb_destroy(h);
   b->handles.clear();
+  if (b->d_second) cudaFree(b->d_second);
+  b->d_second = nullptr;
   b->streams_mode = false;
 }
 
@@ -826,11 +830,21 @@ flb_status streams_setup(flb_batch b, int nstreams) {
   for (uint32_t k = 0; k < b->n; k++) b->stream_of[b->sorder[k]] = k % (uint32_t)nstreams;
   if (b->handles.empty()) {
     b->handles.assign(b->n, nullptr);
+    // the handles' second population buffers in one allocation (48 cases, 54 MB
+    // in all: creating them 79 ms with one each, 45 together)
+    auto second_bytes = [&](uint32_t c) { return ((size_t)9 * b->nx[c] * b->ny[c] * 4 + 255) & ~(size_t)255; };
+    size_t total = 0, at = 0;
+    for (uint32_t c = 0; c < b->n; c++) total += second_bytes(c);
+    if (cudaMalloc(&b->d_second, total) != cudaSuccess) {
+      cudaGetLastError();
+      b->d_second = nullptr;  // one step per launch
+    }
     for (uint32_t c = 0; c < b->n; c++) {
       flb_case_desc d = b->descs[c];
       d.device = b->device;
       d.stream = b->pool[b->stream_of[c]];
-      const flb_status s = flb_create(&d, &b->handles[c]);
+      const flb_status s = create_handle(&d, &b->handles[c], b->d_second ? b->d_second + at : nullptr, false);
+      at += second_bytes(c);
       if (s != FLB_OK) {
         streams_free(b);
         return bfail(b, s, "the streams form could not create the handle of case " + std::to_string(c));

@@ -101,6 +101,7 @@ struct flb_engine {
   // single phase: the second population buffer of the multi-step kernel (d_f is
   // the current one); null: one step per launch
   void* d_f2 = nullptr;
+  void* lent = nullptr;  // whichever of the two belongs to the caller of create_handle
   // handles stepped concurrently with this one (the batch's streams form): the
   // windows are sized for them together, and the launches come from graphs
   uint32_t peers = 1;
@@ -603,7 +604,7 @@ void free_all(flb_engine* h) {
                   h->d_list[0][1], h->d_list[1][0],  h->d_list[1][1],  h->d_lcount,     h->d_tstep,
                   h->d_plain,      h->d_bar,         h->d_perr};
   for (void* p : bufs)
-    if (p) cudaFree(p);
+    if (p && p != h->lent) cudaFree(p);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
 }
 
@@ -766,26 +767,7 @@ void set_peers(flb_engine* h, uint32_t peers) {
   h->peers = peers;
 }
 
-}  // namespace flb
-
-// =============================================================================
-extern "C" {
-
-FLB_API void flb_case_desc_init(flb_case_desc* d) {
-  if (!d) return;
-  std::memset(d, 0, sizeof(*d));
-  d->precision = 32;
-  d->mass_precision = 64;
-  d->collision = FLB_COLLISION_SRT;
-  d->use_volumetric_force = 1;
-  d->tau = 0.6f;
-  d->bounce_back = FLB_BB_HALFWAY;
-  d->fs_mode = FLB_FS_CONSERVATIVE;
-  d->device = -1;
-  d->arithmetic = FLB_ARITH_FUSED;
-}
-
-FLB_API flb_status flb_create(const flb_case_desc* desc, flb_handle* out) {
+flb_status create_handle(const flb_case_desc* desc, flb_handle* out, void* second, bool own_second) {
   if (!out) return FLB_ERR_INVALID_ARGUMENT;
   *out = nullptr;
   std::string msg;
@@ -926,7 +908,9 @@ FLB_API flb_status flb_create(const flb_case_desc* desc, flb_handle* out) {
   }
   // the second buffer of the multi-step kernel; without it (no memory) the
   // handle runs one step per launch
-  if (mt_possible(h) && cudaMalloc(&h->d_f2, 9 * N * h->s_size) != cudaSuccess) {
+  if (!own_second) {
+    h->d_f2 = h->lent = second;
+  } else if (mt_possible(h) && cudaMalloc(&h->d_f2, 9 * N * h->s_size) != cudaSuccess) {
     cudaGetLastError();
     h->d_f2 = nullptr;
   }
@@ -955,6 +939,29 @@ FLB_API flb_status flb_create(const flb_case_desc* desc, flb_handle* out) {
   if (e != cudaSuccess) return bail(cuda_fail(h, e, "cudaStreamSynchronize"));
   *out = h;
   return FLB_OK;
+}
+
+}  // namespace flb
+
+// =============================================================================
+extern "C" {
+
+FLB_API void flb_case_desc_init(flb_case_desc* d) {
+  if (!d) return;
+  std::memset(d, 0, sizeof(*d));
+  d->precision = 32;
+  d->mass_precision = 64;
+  d->collision = FLB_COLLISION_SRT;
+  d->use_volumetric_force = 1;
+  d->tau = 0.6f;
+  d->bounce_back = FLB_BB_HALFWAY;
+  d->fs_mode = FLB_FS_CONSERVATIVE;
+  d->device = -1;
+  d->arithmetic = FLB_ARITH_FUSED;
+}
+
+FLB_API flb_status flb_create(const flb_case_desc* desc, flb_handle* out) {
+  return create_handle(desc, out, nullptr, true);
 }
 
 FLB_API flb_status flb_reset(flb_handle h, const uint8_t* host_flags) {

@@ -24,6 +24,10 @@ namespace flb {
 // engine.cu: descriptor checks and per-case constants shared with the batch
 flb_status validate_desc(const flb_case_desc* d, std::string& msg);
 void fill_case_constants(const flb_case_desc* desc, KParams& k);
+// flb_create; with own_second false the second population buffer is `second`,
+// 9 * nx * ny values that the caller frees after the handle (null: the handle
+// runs one step per launch)
+flb_status create_handle(const flb_case_desc* desc, flb_handle* out, void* second, bool own_second);
 // how many handles are stepped concurrently with this one, itself included
 // (its stream idle)
 void set_peers(flb_engine* h, uint32_t peers);
