@@ -181,7 +181,7 @@ struct Ops {
   // one round of resident blocks, no more than there are super-tiles (blocks
   // without one cost their launch: 64x48 18.2 -> 16.4 us per step)
   static void grids(flb_engine* h, int nsm) {
-    h->grid_sc = std::min(h->ntiles, (uint32_t)(nsm * sc_list_blocks_per_sm<S, C, M>(h->use_vec_list, h->ntiles)));
+    h->grid_sc = std::min(h->ntiles, (uint32_t)(nsm * sc_list_blocks_per_sm<S, C, M>(h->use_vec_list, h->fused, h->ntiles)));
     h->grid_fs1 = std::min(h->ntiles, (uint32_t)(nsm * fs1_blocks_per_sm(h->ntiles)));
     h->grid_fs234 = std::min(h->ntiles, (uint32_t)(nsm * fs234_blocks_per_sm(h->fs_form, h->ntiles)));
   }

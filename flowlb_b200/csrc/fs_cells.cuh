@@ -129,9 +129,9 @@ __device__ __forceinline__ void fs1_cell(const KParams& p, uint32_t x, uint32_t 
 }
 
 // A cell of a deep super-tile: fluid, as all its neighbours, none of them
-// across the grid's edge or a wall.
+// across the grid's edge or a wall.  Returns its mass, which the caller stores.
 template <class S, class C, class M, bool ODD>
-__device__ __forceinline__ void fs1_deep_cell(const KParams& p, uint32_t idx) {
+__device__ __forceinline__ M fs1_deep_cell(const KParams& p, uint32_t idx) {
   const uint32_t nx = p.nx;
   const uint32_t nb[9] = {idx,          idx + 1u,      idx - 1u,      idx + nx,      idx - nx,
                           idx + nx + 1u, idx - nx - 1u, idx - nx + 1u, idx + nx - 1u};
@@ -143,9 +143,8 @@ __device__ __forceinline__ void fs1_deep_cell(const KParams& p, uint32_t idx) {
     in[i + 1] = Codec<S, C>::ld(slotp<S>(p, slot_b<ODD>(i)), nb[i], i + 1, inv);
   }
   load_out<S, C, ODD>(p, idx, nb, out);
-  M* Ms = static_cast<M*>(p.mass);
   const M* Ex = static_cast<const M*>(p.excess);
-  M m = Ms[idx];
+  M m = static_cast<const M*>(p.mass)[idx];
   M exn[9];
 #pragma unroll
   for (int i = 1; i < 9; i++) exn[i] = Ex[nb[i]];
@@ -156,7 +155,7 @@ __device__ __forceinline__ void fs1_deep_cell(const KParams& p, uint32_t idx) {
     m += in[i + 1] - out[i];
     m += in[i] - out[i + 1];
   }
-  Ms[idx] = m;
+  return m;
 }
 
 // ---- FS_2 + FS_3 + FS_4 fused: lbmKernel2D.cu:124-303 ----------------------

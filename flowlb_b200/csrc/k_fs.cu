@@ -10,19 +10,22 @@
 
 namespace flb {
 
-// FS_1 on the listed super-tiles, one row of a super-tile per warp, at 64
-// registers and 1024 threads per SM in either form: two cells per thread
-// (256-thread blocks, four per SM) takes about 500 listed super-tiles in one
-// round; with one cell per thread (512 x 2) the pass is shorter where there are
-// few.  Measured on a B200, us per step with two | one (the flag pass
-// likewise): 101x101 17.2 | 14.9, 300x120 16.4 | 15.0, 1001x401 26.3 | 25.4,
-// 2048x512 24.2 | 27.6, 8192x2048 232 | 264.  The line is kSmallTiles.  At 64
-// registers the FP64 mass arithmetic spills (136 bytes, FP64 storage 350); on
-// grids of up to kTinyTiles super-tiles, whose listed ones fit one block per SM,
-// the one-cell form takes 128: 300x120 14.4 -> 13.4, 601x301 16.2 -> 15.0 (but
-// 1001x401 22.8 -> 24.1; two cells at 85 registers, three blocks per SM:
-// 2048x512 23.4 -> 25.1).
-constexpr int kFs1Block = 256;   // two cells per thread (x and x + 32 of a row), four blocks per SM
+// FS_1 on the listed super-tiles, one row of a super-tile per warp.  With two
+// cells per thread (256-thread blocks, three per SM at 85 registers) about 440
+// listed super-tiles are one round; one cell per thread (512 threads) makes the
+// pass shorter where there are few.  Measured on a B200, us per step with two |
+// one: 101x101 17.2 | 14.9, 300x120 16.4 | 15.0, 1001x401 26.3 | 25.4, 2048x512
+// 24.2 | 27.6, 8192x2048 232 | 264; the line is kSmallTiles.  One cell: two
+// blocks per SM at 64 registers, where the FP64 mass arithmetic spills (136
+// bytes, FP64 storage 350); grids of up to kTinyTiles super-tiles, whose listed
+// ones fit one block per SM, take 128: 300x120 14.4 -> 13.4, 601x301 16.2 -> 15.0
+// (but 1001x401 22.8 -> 24.1).  Two cells, three blocks per SM | four at 64
+// registers | five at 48: 2048x512 FP32 22.4 | 22.5 | 23.6, FP64 25.8 | 26.3 |
+// 31.7, 4001x1201 50.8 | 51.6 | 53.6.  The block's next super-tile is not
+// prefetched into L2: with the short form of the plain-fluid super-tiles that
+// cost more than it hid (8192x2048 FP32 196 against 184, FP16S 183 against 172,
+// 4001x1201 58 against 54).
+constexpr int kFs1Block = 256;   // two cells per thread (x and x + 32 of a row), three blocks per SM
 constexpr int kFs1Small = 512;   // one cell per thread, two blocks per SM, or one
 // lc: the next step's list lengths and marks, cleared here for this step's
 // flag pass.
@@ -35,7 +38,6 @@ __global__ void __launch_bounds__(BLOCK, MB) k_fs1(const __grid_constant__ KPara
   constexpr uint32_t kCpr = BLOCK / 32 / kSTH;         // warps per row of a super-tile
   constexpr uint32_t kCells = kSTW / (32u * kCpr);     // cells per thread and super-tile
   static_assert(kCells * 32u * kCpr == kSTW && kCells <= 2u, "FS_1: one or two cells per thread and super-tile");
-  static_assert(BLOCK >= 118, "FS_1: prefetch_super_tile needs 118 threads");
   // the block's first entry is loaded with the length (the list holds at least
   // a grid of entries, whatever its length)
   uint32_t t = tile_at(tl, blockIdx.x);
@@ -44,16 +46,18 @@ __global__ void __launch_bounds__(BLOCK, MB) k_fs1(const __grid_constant__ KPara
   const uint32_t row = warp % kSTH, chunk = warp / kSTH;
   const uint32_t nx = p.nx;
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x, t = i < n ? tile_at(tl, i) : 0u) {
-    // the block's next super-tile into L2 while this one is worked on
-    if (i + gridDim.x < n) prefetch_super_tile(p, tile_at(tl, i + gridDim.x), tl.nsx, sizeof(S), true, sizeof(M));
     const bool deep = DEEP && (t & kDeepTile);
     t &= ~kDeepTile;
     const uint32_t y = (t / tl.nsx) * kSTH + row;
     if (y >= p.ny) continue;
     const uint32_t xa = (t % tl.nsx) * kSTW + chunk * 32u + lane, xc = xa + 32u * kCpr;
     if (deep) {
+      // the loads of both cells before either store
+      M m[kCells];
 #pragma unroll
-      for (uint32_t k = 0; k < kCells; k++) fs1_deep_cell<S, C, M, ODD>(p, xa + 32u * kCpr * k + y * nx);
+      for (uint32_t k = 0; k < kCells; k++) m[k] = fs1_deep_cell<S, C, M, ODD>(p, xa + 32u * kCpr * k + y * nx);
+#pragma unroll
+      for (uint32_t k = 0; k < kCells; k++) static_cast<M*>(p.mass)[xa + 32u * kCpr * k + y * nx] = m[k];
       continue;
     }
     // the cells' flags and wall masks first: one round trip for both
@@ -103,7 +107,9 @@ __global__ void k_apply_recon(const __grid_constant__ KParams p, uint32_t odd) {
 // per thread two on grids of up to kTinyTiles super-tiles (three spill at 40
 // registers: 300x120 14.4 against 13.4 us per step with FS_1's form), three
 // above (1001x401 22.8 against 23.4); with two cells four (five spill at 48:
-// 2048x512 25.1 against 24.2, 4001x1201 159 against 148).
+// 2048x512 23.5 against 22.5), and five on grids of more than kLargeTiles
+// super-tiles, most of them plain fluid in many rounds (8192x2048 FP32 174
+// against 177, FP16S 168 against 172; 4001x1201 51.6 either way).
 template <class S, class C, class M, bool ODD, int TW, int CPT, int MB, bool THIN>
 __global__ void __launch_bounds__(TW* kTY / CPT, MB)
     k_fs234(const __grid_constant__ KParams p, const TileList tl, uint32_t* __restrict__ nz, const NextLists nl) {
@@ -132,7 +138,7 @@ void launch_fs1(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const
   using std::integral_constant;
   if (tl.ntiles <= kTinyTiles) go(integral_constant<int, kFs1Small>{}, integral_constant<int, 1>{});
   else if (tl.ntiles <= kSmallTiles) go(integral_constant<int, kFs1Small>{}, integral_constant<int, 2>{});
-  else go(integral_constant<int, kFs1Block>{}, integral_constant<int, 4>{});
+  else go(integral_constant<int, kFs1Block>{}, integral_constant<int, 3>{});
 }
 
 template <class S, class C, class M>
@@ -169,15 +175,19 @@ int launch_fs234(const KParams& kp, cudaStream_t st, uint32_t odd, const TileLis
       if (tl.ntiles <= kTinyTiles) launch_fs234_form<S, C, M, 64, 1, 2>(kp, st, odd, tl, grid, nz, nl);
       else launch_fs234_form<S, C, M, 64, 1, 3>(kp, st, odd, tl, grid, nz, nl);
       break;
-    default: launch_fs234_form<S, C, M, 64, 2, 4>(kp, st, odd, tl, grid, nz, nl); break;
+    default:
+      if (tl.ntiles <= kLargeTiles) launch_fs234_form<S, C, M, 64, 2, 4>(kp, st, odd, tl, grid, nz, nl);
+      else launch_fs234_form<S, C, M, 64, 2, 5>(kp, st, odd, tl, grid, nz, nl);
+      break;
   }
   return 1;
 }
 
 // Resident blocks per SM: the launch bounds above.
-int fs1_blocks_per_sm(uint32_t ntiles) { return ntiles <= kTinyTiles ? 1 : ntiles <= kSmallTiles ? 2 : 4; }
+int fs1_blocks_per_sm(uint32_t ntiles) { return ntiles <= kTinyTiles ? 1 : ntiles <= kSmallTiles ? 2 : 3; }
 int fs234_blocks_per_sm(int form, uint32_t ntiles) {
-  return form == FS_FORM_W32 ? 6 : form == FS_FORM_W64X1 ? (ntiles <= kTinyTiles ? 2 : 3) : 4;
+  return form == FS_FORM_W32 ? 6 : form == FS_FORM_W64X1 ? (ntiles <= kTinyTiles ? 2 : 3)
+                               : ntiles <= kLargeTiles ? 4 : 5;
 }
 
 #define FLB_INSTANTIATE(S, C, M)                                                                                  \

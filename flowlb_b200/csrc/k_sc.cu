@@ -59,11 +59,12 @@ __global__ void __launch_bounds__(kBlock, FLB_SC_MIN_BLOCKS) k_sc_scalar(const _
 // 256 x 4 at 64, two cells per thread):
 //   601x301 F32, reference arithmetic  19.5 | 16.0 | 18.1
 //   1001x401 F32  24.8 | 22.8 | 24.4       2048x512 F32  24.3 | 24.0 | 23.7
-//   2048x512 F64  32.0 | 28.4 | 27.6       8192x2048 F32  233 | 242 | 238
-// So: 512 x 2 while the blocks are about one round (kScSmallTiles), 512 x 4
-// where FP32 with the fused arithmetic (few spills at 32 registers) is bound by
-// memory (more than kScLargeTiles super-tiles), 256 x 4 elsewhere.
-constexpr uint32_t kScSmallTiles = 1024, kScLargeTiles = 8192;
+//   2048x512 F64  32.0 | 28.4 | 27.6
+// So: 512 x 2 while the blocks are about one round (kSmallTiles), else 256 x 4,
+// but for FP32 with the fused arithmetic on more than kLargeTiles super-tiles
+// (bound by memory) 512 x 3: 8192x2048 F32 177 us per step against 181 with 256
+// x 4 or 512 x 2, 182 with 256 x 5 and 184 with 512 x 4; 4001x1201 51.6 against
+// 52.7, 51.9, 53.3 and 53.7.
 template <class S, class C, class M, bool HW, bool ODD, bool FU, int BLOCK, int MB, bool DEEP>
 __global__ void __launch_bounds__(BLOCK, MB) k_sc_list(const __grid_constant__ KParams p,
                                                                            const TileList tl) {
@@ -637,6 +638,9 @@ int vec_width(int precision) {
   return precision == 64 ? Lanes<double>::V : (precision == 16 ? Lanes<__half>::V : Lanes<float>::V);
 }
 
+template <class C>
+static bool list_wide(bool fu, uint32_t ntiles) { return fu && sizeof(C) == 4 && ntiles > kLargeTiles; }
+
 template <class S, class C, class M, bool FU>
 static void launch_sc_list_f(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const TileList& tl,
                              uint32_t grid, bool vec) {
@@ -649,13 +653,13 @@ static void launch_sc_list_f(const KParams& kp, cudaStream_t st, uint32_t odd, b
   }
   auto go = [&](auto block, auto mb) {
     constexpr int BLOCK = decltype(block)::value, MB = decltype(mb)::value;
-    constexpr bool DEEP = MB == 4;
+    constexpr bool DEEP = MB != 2;
     if (hw) launch_pdl(k_sc_list<S, C, M, true, false, FU, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl);
     else launch_pdl(k_sc_list<S, C, M, false, false, FU, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl);
   };
   using std::integral_constant;
-  if (tl.ntiles <= kScSmallTiles) go(integral_constant<int, 512>{}, integral_constant<int, 2>{});
-  else if (FU && sizeof(C) == 4 && tl.ntiles > kScLargeTiles) go(integral_constant<int, 512>{}, integral_constant<int, 4>{});
+  if (tl.ntiles <= kSmallTiles) go(integral_constant<int, 512>{}, integral_constant<int, 2>{});
+  else if (list_wide<C>(FU, tl.ntiles)) go(integral_constant<int, 512>{}, integral_constant<int, 3>{});
   else go(integral_constant<int, 256>{}, integral_constant<int, 4>{});
 }
 
@@ -667,8 +671,8 @@ void launch_sc_list(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, c
 }
 
 template <class S, class C, class M>
-int sc_list_blocks_per_sm(bool vec, uint32_t ntiles) {
-  if (!vec) return ntiles <= kScSmallTiles ? 2 : 4;  // the launch bounds
+int sc_list_blocks_per_sm(bool vec, bool fu, uint32_t ntiles) {
+  if (!vec) return ntiles <= kSmallTiles ? 2 : list_wide<C>(fu, ntiles) ? 3 : 4;  // the launch bounds
   int n = 0, m = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sc_list_vec<S, C, M, true, false, false>, list_vec_block<S>(), 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_sc_list_vec<S, C, M, true, false, true>, list_vec_block<S>(), 0);
@@ -680,7 +684,7 @@ int sc_list_blocks_per_sm(bool vec, uint32_t ntiles) {
   template void launch_sc<S, C, M>(const KParams&, cudaStream_t, uint32_t, bool, bool, bool, bool, bool);     \
   template void launch_sc_list<S, C, M>(const KParams&, cudaStream_t, uint32_t, bool, const TileList&, uint32_t,  \
                                         bool, bool);                                                            \
-  template int sc_list_blocks_per_sm<S, C, M>(bool, uint32_t);
+  template int sc_list_blocks_per_sm<S, C, M>(bool, bool, uint32_t);
 FLB_FOR_EACH_VARIANT(FLB_INSTANTIATE)
 #undef FLB_INSTANTIATE
 

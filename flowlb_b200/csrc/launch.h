@@ -46,7 +46,7 @@ template <class S, class C, class M>
 void launch_sc_list(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const TileList& tl, uint32_t grid,
                     bool fu, bool vec);
 template <class S, class C, class M>
-int sc_list_blocks_per_sm(bool vec, uint32_t ntiles);
+int sc_list_blocks_per_sm(bool vec, bool fu, uint32_t ntiles);
 
 // FS_1 (clears the next step's list lengths), its reference-mode apply, and
 // FS_2..4 on listed super-tiles (appends the next step's lists)
@@ -66,8 +66,9 @@ enum FsForm { FS_FORM_W32 = 1, FS_FORM_W64X1 = 5, FS_FORM_W64X2 = 6 };
 int fs1_blocks_per_sm(uint32_t ntiles);
 int fs234_blocks_per_sm(int form, uint32_t ntiles);
 // up to this many super-tiles FS_1 and the flag pass take one cell per thread,
-// up to kTinyTiles FS_1 with all the registers (k_fs.cu)
-constexpr uint32_t kSmallTiles = 1024, kTinyTiles = 512;
+// up to kTinyTiles FS_1 with all the registers (k_fs.cu); above kLargeTiles
+// stream-collide and the flag pass have blocks for many rounds of memory traffic
+constexpr uint32_t kSmallTiles = 1024, kTinyTiles = 512, kLargeTiles = 8192;
 
 // the free-surface step as one persistent cooperative kernel (k_fsp.cu):
 // a.steps steps per launch, `grid` CTAs of 1024 threads all resident at once
