@@ -139,6 +139,9 @@ FLB_API flb_status flb_destroy(flb_handle h);
 
 /* Advances n time steps asynchronously on the handle's stream: per step
  * FS_1, stream-collide, FS_2..4 (free surface) or stream-collide alone.
+ * Single-phase cases without inlet/outlet cells take several steps per launch
+ * between two population buffers where memory for the second one was there at
+ * creation and the stream is not being captured (the same results).
  * Replaces the loop bodies of runCuda.cu:473-490 and :506-527. */
 FLB_API flb_status flb_step(flb_handle h, uint64_t n);
 
@@ -154,7 +157,7 @@ FLB_API flb_status flb_get_time(flb_handle h, uint64_t* t);
  * the flag pass (which lists the next step's super-tiles) as three kernels
  * per step.
  * FLB_STEP_PERSISTENT: one cooperative kernel per graph (every CTA resident,
- * one per SM) runs all its steps, the passes separated by grid barriers in
+ * two per SM) runs all its steps, the passes separated by grid barriers in
  * global memory; a barrier wait gives up after a bounded number of polls
  * (flb_set_wait_limit) and the next flb_sync or flb_read_field returns
  * FLB_ERR_CUDA.  FLB_STEP_AUTO (default): the per-pass kernels, measured
@@ -264,8 +267,8 @@ FLB_API flb_status flb_load_checkpoint(flb_handle h, const char* path);
  * over a pool of streams longest first, and a batch step launches each
  * case's own step graphs on its stream; the cases run concurrently, which
  * hides the per-step launch latency that bounds a per-case loop on one
- * stream.  It keeps a second copy of the state (the handles') and is
- * entered at even steps only.
+ * stream.  It keeps a second copy of the state (the handles', with a
+ * second population buffer each) and is entered at even steps only.
  * autotune: 0 uses 8-CTA clusters, one CTA per SM; 1 (100 probe steps) or a
  * probe step count > 1 times candidate modes, group sizes and counts of the
  * persistent kernel and the streams form with 8 and 16 streams on the batch
