@@ -66,3 +66,39 @@ def test_multi_step_large_grid_equals_one_step_per_launch():
             assert np.array_equal(a.read(fid), b.read(fid)), (prec, fid)
         a.close()
         b.close()
+
+
+def test_inlet_outlet_buffers_over_odd_calls_writes_checkpoint_and_reset(tmp_path):
+    """Inlet/outlet cells read density and velocity of the step before, which
+    two pairs of buffers hold in turn: calls of odd and even lengths, a write-back
+    of both fields, a checkpoint and a reset, against the oracle."""
+    flags = cases.plain_channel(90, 26).flags.copy()
+    flags[1:-1, 0] = cases.INLET
+    flags[1:-1, -1] = cases.OUTLET
+    kw = dict(tau=0.7, inlet_ux=0.04, use_force=False)
+    s, o = pair(flags, O.F32, E.BB_HALFWAY, E.ARITH_FUSED, **kw)
+    for n in (1, 2, 3, 33, 5):
+        s.step(n)
+        o.step(n)
+        check(s, o, O.F32, f"t={o.t}")
+    s.write(E.FIELD_RHO, s.rho)
+    s.write(E.FIELD_U, s.u)
+    s.step(3)
+    o.step(3)
+    check(s, o, O.F32, "after the write-back")
+    path = str(tmp_path / "state.bin")
+    s.save_checkpoint(path)
+    b = E.Solver(flags, precision=32, bounce_back=E.BB_HALFWAY, arithmetic=E.ARITH_FUSED, **kw)
+    b.step(7)
+    b.load_checkpoint(path)
+    for n in (1, 36):
+        b.step(n)
+        o.step(n)
+        check(b, o, O.F32, f"checkpoint, t={o.t}")
+    b.close()
+    s.reset(flags)
+    o = O.Oracle(flags, O.OracleConfig(variant=O.F32, bb=E.BB_HALFWAY, arithmetic=E.ARITH_FUSED, **kw))
+    s.step(35)
+    o.step(35)
+    check(s, o, O.F32, "after the reset")
+    s.close()
