@@ -118,6 +118,11 @@ struct flb_engine {
   void* d_rho_snap = nullptr;
   void* d_u_snap = nullptr;
   bool snap_same = false;  // single phase: the never-written cells hold the same in d_rho, d_u and their snapshots
+  // single phase: the caller has captured a step.  Its graph holds the buffers
+  // of that time and may be replayed between any later calls, so from then on no buffer
+  // changes places: one step per launch in place, density and velocity copied
+  // for the inlet and outlet cells before each
+  bool captured = false;
   double* d_partial = nullptr;
   double* d_scalar = nullptr;
   unsigned long long* d_counts = nullptr;
@@ -305,9 +310,10 @@ uint64_t issue_step(flb_engine* h, uint64_t t, bool write_macro) {
     // cells that are never written hold the same in both; 4001x41 F32 in the
     // reference's modes, 200 steps and the read-back on a B200: 8.8 us per step
     // copying both arrays before every step, 5.3 alternating).  Free surface: which cells are written changes,
-    // so the arrays are copied.
-    if (h->fs || !h->snap_same) copy_snap(h);
-    if (!h->fs) {
+    // so the arrays are copied; so they are once the caller has captured a step.
+    const bool alternate = !h->fs && !h->captured;
+    if (!alternate || !h->snap_same) copy_snap(h);
+    if (alternate) {
       std::swap(h->d_rho, h->d_rho_snap);
       std::swap(h->d_u, h->d_u_snap);
     }
@@ -491,12 +497,20 @@ MtArgs mt_plan(const flb_engine* h, const MtWindow& w, uint64_t left) {
 bool mt_possible(const flb_engine* h) {
   return !h->fs && !h->has_io && h->desc.kernel_variant == 0 && mt_window(h) != nullptr;
 }
-// ... and may now (not while the caller captures the stream: the launch
+// ... and may now (not once the caller has captured a step: the launch
 // alternates between two buffers).
-bool mt_usable(flb_engine* h) {
-  if (!h->d_f2 || !mt_possible(h)) return false;
+bool mt_usable(const flb_engine* h) { return h->d_f2 && !h->captured && mt_possible(h); }
+
+// Single phase: whether the caller is capturing the handle's stream.
+bool caller_captures(flb_engine* h) {
+  if (h->fs) return false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(h->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusActive) return false;
+  if (!h->captured) {
+    h->captured = true;
+    h->g_pair.f = h->g_big.f = nullptr;  // their steps alternate between buffers: captured anew
+  }
+  return true;
 }
 
 // One launch of at most `left` steps, the last of which writes density and
@@ -1011,7 +1025,8 @@ FLB_API flb_status flb_step(flb_handle h, uint64_t n) {
     }
   }
   nvtxRangePushA("flb_step");
-  if (h->has_io && !h->fs && !h->snap_same) copy_snap(h);  // (here: not into a graph of steps)
+  const bool recorded = caller_captures(h);  // every step by itself: a stream in capture cannot be captured again
+  if (h->has_io && !h->fs && !h->captured && !h->snap_same) copy_snap(h);  // (here: not into a graph of steps)
   uint64_t remaining = n;
   flb_status s = FLB_OK;
   if (n >= 2 && mt_usable(h)) {
@@ -1030,7 +1045,7 @@ FLB_API flb_status flb_step(flb_handle h, uint64_t n) {
       h->launches += issue_step(h, h->t, remaining == 1);
       h->t += 1;
       remaining -= 1;
-    } else if ((h->t & 1u) == 0 && remaining >= big + tail) {
+    } else if (!recorded && (h->t & 1u) == 0 && remaining >= big + tail) {
       s = capture(h, h->g_big, kGraphPairs);
       if (s != FLB_OK) break;
       cudaError_t e = cudaGraphLaunch(h->g_big.exec, h->stream);
@@ -1038,7 +1053,7 @@ FLB_API flb_status flb_step(flb_handle h, uint64_t n) {
       h->launches += h->g_big.kernels;
       h->t += big;
       remaining -= big;
-    } else if ((h->t & 1u) == 0 && remaining >= 2 + tail) {
+    } else if (!recorded && (h->t & 1u) == 0 && remaining >= 2 + tail) {
       s = capture(h, h->g_pair, 1);
       if (s != FLB_OK) break;
       cudaError_t e = cudaGraphLaunch(h->g_pair.exec, h->stream);

@@ -141,7 +141,11 @@ FLB_API flb_status flb_destroy(flb_handle h);
  * FS_1, stream-collide, FS_2..4 (free surface) or stream-collide alone.
  * Single-phase cases without inlet/outlet cells take several steps per launch
  * between two population buffers where memory for the second one was there at
- * creation and the stream is not being captured (the same results).
+ * creation (the same results).  A call while the caller captures the handle's
+ * stream is recorded as one kernel per step; the caller may replay it wherever
+ * the step's parity is that of the captured call, between direct calls as well,
+ * so from the first such call on the handle's buffers keep their places and it
+ * takes one step per launch.  flb_get_time does not count replays.
  * Replaces the loop bodies of runCuda.cu:473-490 and :506-527. */
 FLB_API flb_status flb_step(flb_handle h, uint64_t n);
 
