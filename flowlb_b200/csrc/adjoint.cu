@@ -95,7 +95,7 @@ __device__ __forceinline__ Nb sources(uint32_t x, uint32_t y, uint32_t nx, uint3
 
 // Gathers the 9 inputs of a cell from the state fin.
 template <class T>
-__device__ __forceinline__ void gather(const AdjParams<T>& p, const T* __restrict__ fin, uint32_t idx, uint32_t sw,
+__device__ __forceinline__ void gather(const AdjParams<T>& p, const T* fin, uint32_t idx, uint32_t sw,
                                        const Nb& nb, T* f) {
   const uint32_t N = p.N;
   f[0] = fin[idx];
@@ -140,14 +140,17 @@ __device__ __forceinline__ Cell<T> cell_state(const AdjParams<T>& p, const T* f,
 }
 
 
+// No pointer of the two step kernels is __restrict__: while a step's blocks wait
+// (pdl_wait) the step before still writes the arrays that they read next, and
+// the qualifier would let their loads be moved above the wait.
+
 // One forward step fin -> fout (fin null: the segment's checkpoint).  jrow: rho
 // u_x of the last column is added to it.
 // ckpt (segment's first step only): the input state is also copied there.
 template <class T>
 __global__ void __launch_bounds__(kAdjBlock, kAdjFwdBlocks) k_por_fwd(const __grid_constant__ AdjParams<T> p, const T* fin,
-                                                       T* __restrict__ fout, double* __restrict__ jrow,
-                                                       const SegDesc* __restrict__ seg, uint32_t j, int copy_ckpt,
-                                                       T* __restrict__ mac) {
+                                                       T* fout, double* jrow, const SegDesc* seg, uint32_t j,
+                                                       int copy_ckpt, T* mac) {
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   const bool in = x < p.nx;
   const uint32_t idx = in ? x + y * p.nx : 0u, N = p.N;
@@ -207,10 +210,9 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjFwdBlocks) k_por_fwd(const __gr
 // t) (scattered).  sbar: dJ/ds per cell; gpart: dJ/dg per block (2 doubles per
 // block).  The update's derivative needs no population itself, only rho and v.
 template <class T, int MB>
-__global__ void __launch_bounds__(kAdjBlock, MB) k_por_bwd(const __grid_constant__ AdjParams<T> p, const T* __restrict__ mac,
-                                                       const T* __restrict__ lam_next, T* __restrict__ lam,
-                                                       double* __restrict__ sbar, double* __restrict__ gpart,
-                                                       const SegDesc* __restrict__ seg, uint32_t j) {
+__global__ void __launch_bounds__(kAdjBlock, MB) k_por_bwd(const __grid_constant__ AdjParams<T> p, const T* mac,
+                                                       const T* lam_next, T* lam, double* sbar, double* gpart,
+                                                       const SegDesc* seg, uint32_t j) {
   __shared__ double red[2][kAdjBlock / 32];
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   double gxb_d = 0.0, gyb_d = 0.0;

@@ -110,7 +110,9 @@ struct TileList {
 // before its first read of anything the previous kernel wrote (it returns once
 // that kernel has completed and its writes are visible; it returns at once
 // when the kernel was launched without the attribute), then pdl_trigger() to
-// let its own successor be scheduled.
+// let its own successor be scheduled.  Its pointer parameters are not
+// __restrict__: the qualifier says that nothing else writes the array while the
+// kernel runs, and allows a load to be moved above the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
