@@ -830,26 +830,27 @@ flb_status streams_setup(flb_batch b, int nstreams) {
   for (uint32_t k = 0; k < b->n; k++) b->stream_of[b->sorder[k]] = k % (uint32_t)nstreams;
   if (b->handles.empty()) {
     b->handles.assign(b->n, nullptr);
-    // the handles' second population buffers in one allocation (48 cases, 54 MB
-    // in all: creating them 79 ms with one each, 45 together)
-    auto second_bytes = [&](uint32_t c) { return ((size_t)9 * b->nx[c] * b->ny[c] * 4 + 255) & ~(size_t)255; };
-    size_t total = 0, at = 0;
-    for (uint32_t c = 0; c < b->n; c++) total += second_bytes(c);
-    if (cudaMalloc(&b->d_second, total) != cudaSuccess) {
-      cudaGetLastError();
-      b->d_second = nullptr;  // one step per launch
-    }
     for (uint32_t c = 0; c < b->n; c++) {
       flb_case_desc d = b->descs[c];
       d.device = b->device;
       d.stream = b->pool[b->stream_of[c]];
-      const flb_status s = create_handle(&d, &b->handles[c], b->d_second ? b->d_second + at : nullptr, false);
-      at += second_bytes(c);
+      const flb_status s = create_handle(&d, &b->handles[c], false);
       if (s != FLB_OK) {
         streams_free(b);
         return bfail(b, s, "the streams form could not create the handle of case " + std::to_string(c));
       }
     }
+    // then, if there is room, the handles' second population buffers in one
+    // allocation (48 cases, 54 MB in all: creating them 79 ms with one each, 45
+    // together); without it they take one step per launch
+    auto second_bytes = [&](uint32_t c) { return ((size_t)9 * b->nx[c] * b->ny[c] * 4 + 255) & ~(size_t)255; };
+    size_t total = 0, at = 0;
+    for (uint32_t c = 0; c < b->n; c++) total += second_bytes(c);
+    if (cudaMalloc(&b->d_second, total) != cudaSuccess) {
+      cudaGetLastError();
+      b->d_second = nullptr;
+    }
+    for (uint32_t c = 0; b->d_second && c < b->n; at += second_bytes(c++)) lend_second(b->handles[c], b->d_second + at);
   } else {
     for (uint32_t c = 0; c < b->n; c++) {
       const flb_status s = flb_set_stream(b->handles[c], b->pool[b->stream_of[c]]);

@@ -781,7 +781,11 @@ void set_peers(flb_engine* h, uint32_t peers) {
   h->peers = peers;
 }
 
-flb_status create_handle(const flb_case_desc* desc, flb_handle* out, void* second, bool own_second) {
+void lend_second(flb_engine* h, void* second) {
+  if (mt_possible(h)) h->d_f2 = h->lent = second;
+}
+
+flb_status create_handle(const flb_case_desc* desc, flb_handle* out, bool own_second) {
   if (!out) return FLB_ERR_INVALID_ARGUMENT;
   *out = nullptr;
   std::string msg;
@@ -922,9 +926,7 @@ flb_status create_handle(const flb_case_desc* desc, flb_handle* out, void* secon
   }
   // the second buffer of the multi-step kernel; without it (no memory) the
   // handle runs one step per launch
-  if (!own_second) {
-    h->d_f2 = h->lent = second;
-  } else if (mt_possible(h) && cudaMalloc(&h->d_f2, 9 * N * h->s_size) != cudaSuccess) {
+  if (own_second && mt_possible(h) && cudaMalloc(&h->d_f2, 9 * N * h->s_size) != cudaSuccess) {
     cudaGetLastError();
     h->d_f2 = nullptr;
   }
@@ -975,7 +977,7 @@ FLB_API void flb_case_desc_init(flb_case_desc* d) {
 }
 
 FLB_API flb_status flb_create(const flb_case_desc* desc, flb_handle* out) {
-  return create_handle(desc, out, nullptr, true);
+  return create_handle(desc, out, true);
 }
 
 FLB_API flb_status flb_reset(flb_handle h, const uint8_t* host_flags) {

@@ -24,10 +24,11 @@ namespace flb {
 // engine.cu: descriptor checks and per-case constants shared with the batch
 flb_status validate_desc(const flb_case_desc* d, std::string& msg);
 void fill_case_constants(const flb_case_desc* desc, KParams& k);
-// flb_create; with own_second false the second population buffer is `second`,
-// 9 * nx * ny values that the caller frees after the handle (null: the handle
-// runs one step per launch)
-flb_status create_handle(const flb_case_desc* desc, flb_handle* out, void* second, bool own_second);
+// flb_create; with own_second false the handle takes no second population buffer
+// of its own, but may be lent one of 9 * nx * ny values (lend_second) that the
+// caller frees after the handle
+flb_status create_handle(const flb_case_desc* desc, flb_handle* out, bool own_second);
+void lend_second(flb_engine* h, void* second);
 // how many handles are stepped concurrently with this one, itself included
 // (its stream idle)
 void set_peers(flb_engine* h, uint32_t peers);
