@@ -732,7 +732,7 @@ FLB_API flb_status flb_adjoint_create(const flb_adjoint_desc* d, flb_adjoint* ou
                 {(void**)&a->d_gpart, 2 * (size_t)a->nblocks * sizeof(double)},
                 {(void**)&a->d_jrow, a->ny * sizeof(double)}, {(void**)&a->d_seg, 2 * sizeof(SegDesc)}};
   for (Al& x : allocs) {
-    cudaError_t e = cudaMalloc(x.p, x.bytes);
+    cudaError_t e = with_spare([&] { return cudaMalloc(x.p, x.bytes); });
     if (e != cudaSuccess) return bail(afail(a, FLB_ERR_OUT_OF_MEMORY, "cudaMalloc"));
   }
   if (cudaStreamCreateWithFlags(&a->side, cudaStreamNonBlocking) != cudaSuccess ||

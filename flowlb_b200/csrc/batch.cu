@@ -638,7 +638,7 @@ flb_status bassign(flb_batch b, int clusters) {
   // the new arrays are complete before the old ones go, so a failure leaves
   // the previous assignment in place
   uint32_t* d_start = nullptr;
-  FLB_BCUDA(b, cudaMalloc(&d_start, start.size() * sizeof(uint32_t)));
+  FLB_BCUDA(b, with_spare([&] { return cudaMalloc(&d_start, start.size() * sizeof(uint32_t)); }));
   // stream-ordered copies (the batch's stream is non-blocking, and a plain
   // cudaMemcpy from pageable memory may return before its data land), waited
   // for before the host arrays go out of scope
@@ -846,10 +846,7 @@ flb_status streams_setup(flb_batch b, int nstreams) {
     auto second_bytes = [&](uint32_t c) { return ((size_t)9 * b->nx[c] * b->ny[c] * 4 + 255) & ~(size_t)255; };
     size_t total = 0, at = 0;
     for (uint32_t c = 0; c < b->n; c++) total += second_bytes(c);
-    if (cudaMalloc(&b->d_second, total) != cudaSuccess) {
-      cudaGetLastError();
-      b->d_second = nullptr;
-    }
+    b->d_second = static_cast<char*>(optional_buffer(total));
     for (uint32_t c = 0; b->d_second && c < b->n; at += second_bytes(c++)) lend_second(b->handles[c], b->d_second + at);
   } else {
     for (uint32_t c = 0; c < b->n; c++) {
@@ -1179,7 +1176,7 @@ FLB_API flb_status flb_batch_create(const flb_case_desc* cases, uint32_t n, int 
   };
   for (A& a : allocs) {
     if (!a.need) continue;
-    cudaError_t e = cudaMalloc(a.p, a.bytes);
+    cudaError_t e = with_spare([&] { return cudaMalloc(a.p, a.bytes); });
     if (e != cudaSuccess) return bail(bcuda(b, e, "cudaMalloc"));
   }
   b->hcases.resize(n);

@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <type_traits>
 #include <utility>
@@ -99,9 +100,14 @@ struct flb_engine {
   // device buffers
   void* d_f = nullptr;
   // single phase: the second population buffer of the multi-step kernel (d_f is
-  // the current one); null: one step per launch
+  // the current one); null: one step per launch.  Taken by the first call of two
+  // steps or more (take_second), given back when memory runs out (release_spare)
   void* d_f2 = nullptr;
-  void* lent = nullptr;  // whichever of the two belongs to the caller of create_handle
+  bool own_second = true;  // false: a buffer of the batch's, or none
+  void* lent = nullptr;    // whichever of the two is the batch's
+  std::mutex second_mu;    // held by a call that uses the second buffer
+  flb_engine* next_holder = nullptr;
+  uint32_t second_wait = 0;  // calls until it is asked for again
   // handles stepped concurrently with this one (the batch's streams form): the
   // windows are sized for them together, and the launches come from graphs
   uint32_t peers = 1;
@@ -497,9 +503,59 @@ MtArgs mt_plan(const flb_engine* h, const MtWindow& w, uint64_t left) {
 bool mt_possible(const flb_engine* h) {
   return !h->fs && !h->has_io && h->desc.kernel_variant == 0 && mt_window(h) != nullptr;
 }
-// ... and may now (not once the caller has captured a step: the launch
-// alternates between two buffers).
-bool mt_usable(const flb_engine* h) { return h->d_f2 && !h->captured && mt_possible(h); }
+
+// Failure injection on the host: FLB_FAIL_ALLOC_AT=second in the environment
+// fails the second population buffers, as cudaMalloc does when memory runs out.
+bool fail_second() {
+  const char* v = std::getenv("FLB_FAIL_ALLOC_AT");
+  return v && !std::strcmp(v, "second");
+}
+
+// Another stream of the program may be in capture, which an allocation would
+// otherwise break.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// The handles that own a second buffer, of every device (a list through
+// next_holder).  Never destroyed: a program may destroy its handles at exit.
+struct Holders {
+  std::mutex mu;
+  flb_engine* first = nullptr;
+};
+Holders& holders() {
+  static Holders* const h = new Holders;
+  return *h;
+}
+
+// Takes the second buffer, or leaves the handle without: it is a convenience,
+// so it never takes more than half of what is free.  Where it was refused or
+// given back it is asked for again 64 calls later (asking costs 70 us).
+constexpr uint32_t kSecondWait = 64;
+bool take_second(flb_engine* h) {
+  if (h->second_wait > 0 && --h->second_wait > 0) return false;
+  const size_t bytes = 9ull * h->N * h->s_size;
+  void* p = optional_buffer(bytes);
+  if (!p) {
+    h->second_wait = kSecondWait;
+    return false;
+  }
+  Holders& hs = holders();
+  std::lock_guard<std::mutex> lk(hs.mu);
+  h->d_f2 = p;
+  h->next_holder = hs.first;
+  hs.first = h;
+  return true;
+}
+
+// Whether this call's steps run several to a launch (h->second_mu held).  Not
+// once the caller has captured a step: the launch alternates between two buffers.
+bool mt_usable(flb_engine* h) {
+  if (h->captured || !mt_possible(h)) return false;
+  return h->d_f2 || (h->own_second && take_second(h));
+}
 
 // Single phase: whether the caller is capturing the handle's stream.
 bool caller_captures(flb_engine* h) {
@@ -608,6 +664,15 @@ flb_status check_persist(flb_engine* h) {
 }
 
 void free_all(flb_engine* h) {
+  {
+    Holders& hs = holders();
+    std::lock_guard<std::mutex> lk(hs.mu);
+    for (flb_engine** p = &hs.first; *p; p = &(*p)->next_holder)
+      if (*p == h) {
+        *p = h->next_holder;
+        break;
+      }
+  }
   for (GraphSlot& g : h->g_mt) destroy_graph(g);
   destroy_graph(h->g_pair);
   destroy_graph(h->g_big);
@@ -703,7 +768,7 @@ flb_status initialise(flb_engine* h) {
 template <class Launch>
 flb_status viz_run(flb_handle h, size_t bytes, void* dst, int on_device, Launch&& launch) {
   uint8_t* out = static_cast<uint8_t*>(dst);
-  if (!on_device) FLB_CUDA(h, cudaMallocAsync((void**)&out, bytes, h->stream));
+  if (!on_device) FLB_CUDA(h, with_spare([&] { return cudaMallocAsync((void**)&out, bytes, h->stream); }));
   launch(out);
   h->launches++;
   cudaError_t e = cudaGetLastError();
@@ -775,6 +840,44 @@ void fill_case_constants(const flb_case_desc* desc, KParams& k) {
 
 flb_status validate_desc(const flb_case_desc* d, std::string& msg) { return validate(d, msg); }
 
+void* optional_buffer(size_t bytes) {
+  RelaxedCapture relaxed;
+  size_t free_bytes = 0, total = 0;
+  void* p = nullptr;
+  if (!fail_second() && cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && bytes <= free_bytes / 2 &&
+      cudaMalloc(&p, bytes) == cudaSuccess)
+    return p;
+  cudaGetLastError();
+  return nullptr;
+}
+
+bool release_spare() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  RelaxedCapture relaxed;
+  bool any = false;
+  Holders& hs = holders();
+  std::lock_guard<std::mutex> lk(hs.mu);
+  for (flb_engine** p = &hs.first; *p;) {
+    flb_engine* h = *p;
+    std::unique_lock<std::mutex> use(h->second_mu, std::try_to_lock);
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    // its last launches may still read the buffer: wait for them
+    if (h->device == dev && use.owns_lock() && cudaStreamIsCapturing(h->stream, &cs) == cudaSuccess &&
+        cs == cudaStreamCaptureStatusNone && cudaStreamSynchronize(h->stream) == cudaSuccess &&
+        cudaFree(h->d_f2) == cudaSuccess) {
+      h->d_f2 = nullptr;
+      h->second_wait = kSecondWait;
+      *p = h->next_holder;
+      any = true;
+    } else {
+      p = &h->next_holder;
+    }
+  }
+  cudaGetLastError();
+  return any;
+}
+
 void set_peers(flb_engine* h, uint32_t peers) {
   if (h->peers == peers) return;
   for (GraphSlot& g : h->g_mt) destroy_graph(g);
@@ -804,6 +907,7 @@ flb_status create_handle(const flb_case_desc* desc, flb_handle* out, bool own_se
   h->N = desc->nx * desc->ny;
   h->fs = desc->free_surface != 0;
   h->hw = desc->bounce_back == FLB_BB_HALFWAY;
+  h->own_second = own_second;
   h->fused = desc->arithmetic == FLB_ARITH_FUSED && desc->collision == FLB_COLLISION_SRT && !desc->subgrid;
   if (desc->device >= 0) h->device = desc->device;
   else cudaGetDevice(&h->device);
@@ -914,21 +1018,19 @@ flb_status create_handle(const flb_case_desc* desc, flb_handle* out, bool own_se
   };
   // Failure injection on the host: with FLB_FAIL_ALLOC_AT=k in the
   // environment the k-th device allocation of this creation fails as
-  // cudaMalloc does when memory runs out (nothing is allocated for it), so the
-  // clean-up path can be exercised without exhausting a GPU.
+  // cudaMalloc does when memory runs out (nothing is allocated for it, unless
+  // other handles then give a buffer back), so the clean-up path can be
+  // exercised without exhausting a GPU.
   long fail_at = 0;
   if (const char* v = std::getenv("FLB_FAIL_ALLOC_AT")) fail_at = std::strtol(v, nullptr, 10);
   long nalloc = 0;
   for (Alloc& a : allocs) {
     if (!a.need) continue;
-    cudaError_t e = ++nalloc == fail_at ? cudaErrorMemoryAllocation : cudaMalloc(a.p, a.bytes);
+    bool injected = ++nalloc == fail_at;
+    const cudaError_t e = with_spare([&] {
+      return std::exchange(injected, false) ? cudaErrorMemoryAllocation : cudaMalloc(a.p, a.bytes);
+    });
     if (e != cudaSuccess) return bail(cuda_fail(h, e, "cudaMalloc"));
-  }
-  // the second buffer of the multi-step kernel; without it (no memory) the
-  // handle runs one step per launch
-  if (own_second && mt_possible(h) && cudaMalloc(&h->d_f2, 9 * N * h->s_size) != cudaSuccess) {
-    cudaGetLastError();
-    h->d_f2 = nullptr;
   }
   if (h->fs) {
     // list lengths start at zero
@@ -1031,9 +1133,12 @@ FLB_API flb_status flb_step(flb_handle h, uint64_t n) {
   if (h->has_io && !h->fs && !h->captured && !h->snap_same) copy_snap(h);  // (here: not into a graph of steps)
   uint64_t remaining = n;
   flb_status s = FLB_OK;
-  if (n >= 2 && mt_usable(h)) {
-    s = mt_steps(h, n);
-    remaining = 0;
+  if (n >= 2) {
+    std::lock_guard<std::mutex> lk(h->second_mu);
+    if (mt_usable(h)) {
+      s = mt_steps(h, n);
+      remaining = 0;
+    }
   }
   while (remaining > 0 && s == FLB_OK) {
     // graphs cover pairs of steps from an even t; the last step of the call
@@ -1132,6 +1237,7 @@ FLB_API flb_status flb_set_stream(flb_handle h, void* stream) {
   if (!h) return FLB_ERR_INVALID_ARGUMENT;
   DeviceGuard guard(h->device);
   FLB_CUDA(h, cudaStreamSynchronize(h->stream));
+  std::lock_guard<std::mutex> lk(h->second_mu);  // (release_spare waits for the stream)
   if (h->own_stream) cudaStreamDestroy(h->stream);
   if (stream) {
     h->stream = static_cast<cudaStream_t>(stream);
@@ -1195,7 +1301,7 @@ FLB_API flb_status flb_read_field(flb_handle h, int field, void* dst, int on_dev
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   if (field == FLB_FIELD_F && h->variant == V_F16S) {
     void* tmp = nullptr;
-    FLB_CUDA(h, cudaMallocAsync(&tmp, bytes, h->stream));
+    FLB_CUDA(h, with_spare([&] { return cudaMallocAsync(&tmp, bytes, h->stream); }));
     refresh_params(h);
     dispatch(h, [&](auto ops) { ops.decode(h, tmp); });
     h->launches++;
@@ -1219,7 +1325,7 @@ FLB_API flb_status flb_write_field(flb_handle h, int field, const void* src, int
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   if (field == FLB_FIELD_F && h->variant == V_F16S) {
     void* tmp = nullptr;
-    FLB_CUDA(h, cudaMallocAsync(&tmp, bytes, h->stream));
+    FLB_CUDA(h, with_spare([&] { return cudaMallocAsync(&tmp, bytes, h->stream); }));
     cudaError_t e = cudaMemcpyAsync(tmp, src, bytes, kind, h->stream);
     if (e == cudaSuccess) {
       refresh_params(h);
@@ -1262,7 +1368,7 @@ FLB_API flb_status flb_viz_shade(flb_handle h, int quantity, const float* colorm
   DeviceGuard guard(h->device);
   float* cmap = nullptr;
   const size_t cbytes = 3 * sizeof(float) * (size_t)n_colors;
-  FLB_CUDA(h, cudaMallocAsync((void**)&cmap, cbytes, h->stream));
+  FLB_CUDA(h, with_spare([&] { return cudaMallocAsync((void**)&cmap, cbytes, h->stream); }));
   cudaError_t e = cudaMemcpyAsync(cmap, colormap_rgb, cbytes, cudaMemcpyHostToDevice, h->stream);
   if (e != cudaSuccess) {
     cudaFreeAsync(cmap, h->stream);

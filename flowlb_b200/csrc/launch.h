@@ -29,6 +29,21 @@ void fill_case_constants(const flb_case_desc* desc, KParams& k);
 // caller frees after the handle
 flb_status create_handle(const flb_case_desc* desc, flb_handle* out, bool own_second);
 void lend_second(flb_engine* h, void* second);
+// memory that is not needed but makes steps faster: at most half of what is free
+// on the current device; null: none
+void* optional_buffer(size_t bytes);
+// gives back, on the current device, the handles' second population buffers that
+// no call is using; whether there was one.  Those handles take one again when
+// there is room.
+bool release_spare();
+// an allocation that, when memory runs out, is tried again after release_spare
+template <class Alloc>
+cudaError_t with_spare(Alloc&& alloc) {
+  cudaError_t e = alloc();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  return release_spare() ? alloc() : e;
+}
 // how many handles are stepped concurrently with this one, itself included
 // (its stream idle)
 void set_peers(flb_engine* h, uint32_t peers);

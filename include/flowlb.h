@@ -140,8 +140,10 @@ FLB_API flb_status flb_destroy(flb_handle h);
 /* Advances n time steps asynchronously on the handle's stream: per step
  * FS_1, stream-collide, FS_2..4 (free surface) or stream-collide alone.
  * Single-phase cases without inlet/outlet cells take several steps per launch
- * between two population buffers where memory for the second one was there at
- * creation (the same results).  A call while the caller captures the handle's
+ * between two population buffers (the same results).  The first call of two steps
+ * or more takes the second one if it is at most half of the free memory, and the
+ * library gives those of idle handles back when an allocation of its own runs
+ * out of memory.  A call while the caller captures the handle's
  * stream is recorded as one kernel per step; the caller may replay it wherever
  * the step's parity is that of the captured call, between direct calls as well,
  * so from the first such call on the handle's buffers keep their places and it
