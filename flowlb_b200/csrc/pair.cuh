@@ -52,10 +52,12 @@ __device__ __forceinline__ void st_pair(float* q, f2 a) { *reinterpret_cast<unsi
 
 // -1/x of both halves, each the correctly rounded quotient (the negative of
 // what __frcp_rn returns).  x away from the ends of the exponent range: the hardware's
-// approximation, within an ulp, and one Newton step with the residual taken in
-// a fused multiply-add, which rounds the exact quotient correctly (Markstein,
-// IBM J. Res. Dev. 34, 1990; here checked against __frcp_rn for every float).
-// Otherwise __frcp_rn itself.
+// approximation and one Newton step with the residual taken in a fused
+// multiply-add (Markstein, IBM J. Res. Dev. 34, 1990).  His theorem has the step
+// round the quotient correctly if the starting value is within an ulp of it and
+// the significand of x is not all ones; that the approximation serves, and for
+// those x too, is tested against __frcp_rn for every float in either half
+// (tests/test_gpu_pair_rcp.py).  Otherwise __frcp_rn itself.
 __device__ __forceinline__ f2 neg_rcp(f2 x) {
   // biased exponents in [2, 251]: neither x nor 1/x is subnormal, zero, infinite or NaN
   const uint32_t ea = __float_as_uint(lo(x)) << 1, eb = __float_as_uint(hi(x)) << 1;
