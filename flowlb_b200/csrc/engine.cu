@@ -439,47 +439,123 @@ flb_status capture(flb_engine* h, GraphSlot& g, int pairs) {
 
 // ---- single phase: several steps per launch (k_mt.cu) -----------------------
 // The window sizes a grid may use: steps per launch, window columns and rows,
-// threads, and packed pairs or one cell per thread.  On small grids the launch
-// is one round of windows and its latency is what counts, so the windows are
-// small (more of them, more recomputed cells) and take many steps; on large
-// grids the recomputed cells count, so the windows are as large as still lets
-// three (FP64: two) run per SM.  Measured on a B200 in us per step, old = one
-// step per launch (grid, storage: old | small windows ... large ones):
-//   256x64    F32 4.1 | 8 x 32x24: 1.05    4 x 32x24: 1.5     4 x 64x22: 2.2
-//   512x160   F32 4.0 | 2.8                1.79               6 x 64x32: 2.2   4 x 64x22: 2.2
-//   1024x256  F32 4.6 | 6.9                3.9                2.9              3.9
-//   1400x360  F32 8.7 | 12.8               6.7                5.1              4.9
-//   4096x1024 F32 50  | 106                52                 34               28.5
-//   1025x256  F64 8.5 | 14                 7.9                5.2              6.2
-//   4097x1024 F64 114 | 231                123                73               66
-//   1025x256  F16 5.6 | 16                 7.9                4.9              5.2
-//   4096x1024 F16 27  | 243                111                53               42
-// FP16 storage above 300,000 cells and FP32 with the reference arithmetic above
-// 110,000 (1024x256: 5.8 | 5.5; 2048x512: 15.8 | 17.1) stay at one step per launch.
+// threads, and packed pairs or one cell per thread; no steps: one step per
+// launch.  On small grids the launch is one round of windows and its latency is
+// what counts, so the windows are small (more of them, more recomputed cells)
+// and take many steps; on large grids the recomputed cells count, so the windows
+// are as large as still lets three (FP64: two) run per SM.  Between them the
+// time goes in rounds of one or two windows per SM, which is what the limits on
+// the number of windows are for.  Channels of a few rows fill few rows of a
+// window.  A call takes the first row of its table that admits it.
+//
+// Measured on a B200, us per step in calls of 100 (one step per launch | the
+// windows on either side of a line, A = 8 steps on 32x24, B = 4 on 32x24, C = 6 on
+// 64x32 or 64x28, D = 4 on 64x22), for rows of whole vectors of four cells unless
+// the width is odd:
+//  FP32, fused arithmetic
+//   131x130 2.4 | A 1.3, B 1.7    136x138 4.4 | A 1.2, B 1.5    212x212 4.0 | A 1.8, B 1.6
+//   328x329 4.3 | B 1.8, C 2.3    676x169 4.4 | B 2.5, C 2.1    336x339 4.3 | B 2.3, C 2.4
+//   1248x312 7.5 | C 4.1, D 3.9   648x648 6.3 | C 4.7, D 4.0    8192x2048 182 | D 107
+//   few rows: 25000x4 4.7 | B 4.0, C 2.3, D 1.8   33332x3 4.6 | B 4.9, C 2.6, D 1.8
+//             66665x3 3.1 | C 4.2, D 3.2          500000x3 9.3 | C 33, D 18
+//  FP32, reference arithmetic
+//   155x155 2.9 | A 2.2, B 2.4    165x164 3.0 | A 2.3, B 2.5    268x268 4.2 | B 3.0, C 3.0
+//   632x158 3.8 | B 3.0, C 3.0    1315x82 4.2 | B 3.6, C 3.1    64x1562 4.9 | B 3.0, C 5.3
+//   676x169 4.1 | B 4.3, C 5.1    384x387 4.9 | B 4.5, C 5.2    16664x6 3.4 | B 4.1, C 4.4
+//  FP32, TRT (subgrid model: within 10% of these)
+//   192x192 3.2 | A 2.7, B 3.0    256x256 3.1 | A 4.9, B 3.5    995x62 3.5 | B 3.6
+//   1872x32 3.3 | A 4.6, B 3.4    300x200 4.0 | A 4.9, B 3.5 (the one grid of six by the line that loses)
+//   640x120 3.8 | B 3.5, C 3.7    384x256 4.2 | B 3.7, C 3.6    4164x24 4.0 | B 4.4, C 4.5
+//   512x256 4.2 | B 5.8, C 6.4
+//  FP64
+//   131x130 3.0 | A 1.8, B 2.0    149x148 3.1 | A 2.1, B 2.0    480x120 3.3 | B 2.5, C 3.3, D 3.3
+//   248x249 3.7 | B 3.5, D 3.3    256x256 3.1 | B 3.5, C 3.4, D 3.3   1073x67 4.1 | B 3.2, C 2.8, D 3.0
+//   1248x312 9.5 | C 8.5, D 8.6   1128x282 8.7 | C 8.3, D 6.8   8192x2048 426 | D 270
+//   64x4531 8.5 | C 9.4, D 8.7    few rows: 16664x6 3.8 | C 3.9, D 3.1   50001x3 4.2 | C 5.8, D 4.2
+//             100000x4 7.8 | C 17, D 10
+//  FP16 storage
+//   260x65 5.1 | A 1.9, B 1.7     480x120 5.7 | B 2.5, C 2.8    496x124 5.7 | B 2.8, C 2.8
+//   1056x264 7.3 | C 4.2          1128x282 6.8 | C 6.2          8192x2048 108 | C above 240
+//   odd rows: 213x212 2.9 | B 1.9, C 3.2   963x60 2.9 | B 3.0, C 3.1   269x268 3.5 | B 3.2, C 3.3
+//             1357x84 3.5 | C 3.1          1549x96 3.8 | C 4.6         1023x255 4.7 | C 4.9
+//             529x529 5.8 | C 4.9
+//   few rows: 33332x3 5.6 | C 3.2          60000x5 6.3 | C 6.9
+//
+// A call of fewer than 34 steps has no graph of 32 one-step launches to compete
+// with (256x256 FP64: 4.2 us per step in calls of 20, 3.1 in calls of 100) and
+// takes the first table, where only the line to one step per launch counts:
+// calls of two steps, us (one step per launch | windows): FP64 512x512 19 | C 24,
+// 469x469 20 | C 12; odd FP16 995x62 8 | B 6, C 11, 1549x96 11 | C 13.
 struct MtWindow {
-  uint64_t cells;  // for grids of up to this many cells
+  uint64_t cells;    // for grids of up to this many cells ...
+  int tiles, few;    // ... that it cuts into up to so many windows, with fewer than kFewRows rows so many ...
+  int only;          // ... see below
   int T, W, H, threads, pairs;
 };
+enum MtOnly {
+  MT_ALL = 0,
+  MT_NARROW = 1,  // a grid narrower than kNarrow needs not keep the limit (one step per launch is as slow there)
+  MT_WHOLE = 2,   // only rows of whole warps, on which one step per launch is at its best
+  MT_WIDE = 4     // only grids that are not narrow
+};
 constexpr uint64_t kAnyCells = ~0ull;
-constexpr MtWindow kMtF32[] = {{18000, 8, 32, 24, 384, 1}, {110000, 4, 32, 24, 384, 1}, {400000, 6, 64, 32, 512, 1},
-                               {kAnyCells, 4, 64, 22, 256, 1}};
-constexpr MtWindow kMtF32Ref[] = {{25000, 8, 32, 24, 384, 0}, {75000, 4, 32, 24, 384, 0}, {110000, 6, 64, 28, 896, 0}};
-constexpr MtWindow kMtF64[] = {{18000, 8, 32, 24, 512, 0}, {75000, 4, 32, 24, 512, 0}, {400000, 6, 64, 32, 512, 0},
-                               {kAnyCells, 4, 64, 22, 256, 0}};
-constexpr MtWindow kMtF16[] = {{18000, 8, 32, 24, 768, 0}, {60000, 4, 32, 24, 768, 0}, {300000, 6, 64, 32, 512, 0}};
-
-template <size_t n>
-const MtWindow* mt_pick(const MtWindow (&w)[n], uint64_t cells) {
-  for (const MtWindow& x : w)
-    if (cells <= x.cells) return &x;
-  return nullptr;
-}
-const MtWindow* mt_window(const flb_engine* h) {
-  const uint64_t cells = (uint64_t)h->N * h->peers;
-  if (h->s_size == 8) return mt_pick(kMtF64, cells);
-  if (h->s_size == 2) return mt_pick(kMtF16, cells);
-  return h->fused ? mt_pick(kMtF32, cells) : mt_pick(kMtF32Ref, cells);
-}
+constexpr int kAnyTiles = 0x7fffffff;
+constexpr uint32_t kFewRows = 8, kNarrow = 49;
+constexpr uint64_t kLongCall = 34;  // 32 steps and the two that are not in a graph with them
+#define FLB_MT_A(threads, pairs) 8, 32, 24, threads, pairs
+#define FLB_MT_B(threads, pairs) 4, 32, 24, threads, pairs
+#define FLB_MT_C(threads, pairs) 6, 64, 32, threads, pairs
+#define FLB_MT_D(threads, pairs) 4, 64, 22, threads, pairs
+#define FLB_MT_ONE 0, 0, 0, 0, 0
+constexpr MtWindow kMtF32[] = {{18000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(384, 1)},
+                               {110000, 350, 350, MT_NARROW, FLB_MT_B(384, 1)},
+                               {400000, 520, 520, MT_NARROW, FLB_MT_C(512, 1)},
+                               {kAnyCells, kAnyTiles, 600, MT_ALL, FLB_MT_D(256, 1)}};
+constexpr MtWindow kMtF32Ref[] = {{25000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(384, 0)},
+                                  {75000, 296, 296, MT_NARROW, FLB_MT_B(384, 0)},
+                                  {110000, 160, 160, MT_ALL, 6, 64, 28, 896, 0},
+                                  {110000, 296, 296, MT_NARROW, FLB_MT_B(384, 0)}};
+// TRT or the subgrid model
+constexpr MtWindow kMtF32Dear[] = {{37000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(384, 0)},
+                                   {55000, 296, 296, MT_NARROW, FLB_MT_B(384, 0)},
+                                   {70000, kAnyTiles, kAnyTiles, MT_WIDE, FLB_MT_ONE},
+                                   {75000, 296, 296, MT_NARROW, FLB_MT_B(384, 0)},
+                                   {110000, 148, 148, MT_ALL, 6, 64, 28, 896, 0},
+                                   {110000, 296, 296, MT_NARROW, FLB_MT_B(384, 0)}};
+constexpr MtWindow kMtF64[] = {{18000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(512, 0)},
+                               {58000, 296, 296, MT_ALL, FLB_MT_B(512, 0)},
+                               {70000, kAnyTiles, kAnyTiles, MT_WHOLE, FLB_MT_ONE},
+                               {70000, kAnyTiles, 600, MT_ALL, FLB_MT_D(256, 0)},
+                               {400000, 355, 355, MT_ALL, FLB_MT_C(512, 0)},
+                               {kAnyCells, kAnyTiles, 600, MT_ALL, FLB_MT_D(256, 0)}};
+constexpr MtWindow kMtF16[] = {{18000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(768, 0)},
+                               {60000, 340, 340, MT_NARROW, FLB_MT_B(768, 0)},
+                               {300000, 1100, 1100, MT_NARROW, FLB_MT_C(512, 0)}};
+// rows that are not whole vectors: 2-byte loads and stores
+constexpr MtWindow kMtF16Odd[] = {{18000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(768, 0)},
+                                  {50000, 296, 296, MT_ALL, FLB_MT_B(768, 0)},
+                                  {70000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_ONE},
+                                  {300000, 148, 148, MT_ALL, FLB_MT_C(512, 0)},
+                                  {270000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_ONE},
+                                  {300000, 300, 300, MT_ALL, FLB_MT_C(512, 0)}};
+// calls of fewer than kLongCall steps
+constexpr MtWindow kMtF32Short[] = {{18000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(384, 1)},
+                                    {110000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_B(384, 1)},
+                                    {400000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_C(512, 1)},
+                                    {kAnyCells, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_D(256, 1)}};
+constexpr MtWindow kMtF32RefShort[] = {{25000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(384, 0)},
+                                       {75000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_B(384, 0)},
+                                       {110000, kAnyTiles, kAnyTiles, MT_ALL, 6, 64, 28, 896, 0}};
+constexpr MtWindow kMtF64Short[] = {{18000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(512, 0)},
+                                    {75000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_B(512, 0)},
+                                    {400000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_C(512, 0)},
+                                    {kAnyCells, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_D(256, 0)}};
+constexpr MtWindow kMtF16Short[] = {{18000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(768, 0)},
+                                    {60000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_B(768, 0)},
+                                    {300000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_C(512, 0)}};
+constexpr MtWindow kMtF16OddShort[] = {{18000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(768, 0)},
+                                       {80000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_B(768, 0)},
+                                       {300000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_C(512, 0)}};
 
 // The launch of at most `left` steps (a.T of them) on windows w.
 MtArgs mt_plan(const flb_engine* h, const MtWindow& w, uint64_t left) {
@@ -499,10 +575,41 @@ MtArgs mt_plan(const flb_engine* h, const MtWindow& w, uint64_t left) {
   return a;
 }
 
-// Whether this handle's steps can run several to a launch.
-bool mt_possible(const flb_engine* h) {
-  return !h->fs && !h->has_io && h->desc.kernel_variant == 0 && mt_window(h) != nullptr;
+template <size_t n>
+const MtWindow* mt_pick(const MtWindow (&table)[n], const flb_engine* h, uint64_t cells) {
+  const bool narrow = h->nx < kNarrow, whole = !narrow && h->nx % 32u == 0;
+  for (const MtWindow& w : table) {
+    if (cells > w.cells || (w.only == MT_WHOLE && !whole) || (w.only == MT_WIDE && narrow)) continue;
+    if (w.T == 0) return nullptr;
+    const uint64_t tiles = (uint64_t)mt_plan(h, w, (uint64_t)w.T).tiles * h->peers;
+    if (tiles <= (uint64_t)(h->ny < kFewRows ? w.few : w.tiles) || (w.only == MT_NARROW && narrow)) return &w;
+  }
+  return nullptr;
 }
+
+// The windows on which a call of n steps runs several to a launch, or null.
+const MtWindow* mt_window(const flb_engine* h, uint64_t n) {
+  if (h->fs || h->has_io || h->desc.kernel_variant != 0 || n < 2) return nullptr;
+  const uint64_t cells = (uint64_t)h->N * h->peers;
+  const bool narrow = h->nx < kNarrow, odd = h->nx % 4u != 0;
+  if (n >= kLongCall || narrow || h->ny < 2u * kFewRows) {
+    if (h->s_size == 8) return mt_pick(kMtF64, h, cells);
+    if (h->s_size == 2) return odd && !narrow ? mt_pick(kMtF16Odd, h, cells) : mt_pick(kMtF16, h, cells);
+    if (h->fused) return mt_pick(kMtF32, h, cells);
+    return h->desc.collision == FLB_COLLISION_SRT && !h->desc.subgrid ? mt_pick(kMtF32Ref, h, cells)
+                                                                       : mt_pick(kMtF32Dear, h, cells);
+  }
+  const MtWindow* w = h->s_size == 8   ? mt_pick(kMtF64Short, h, cells)
+                      : h->s_size == 2 ? (odd ? mt_pick(kMtF16OddShort, h, cells) : mt_pick(kMtF16Short, h, cells))
+                      : h->fused       ? mt_pick(kMtF32Short, h, cells)
+                                       : mt_pick(kMtF32RefShort, h, cells);
+  // two steps on six-step windows: the recomputed border is not paid back
+  if (w && n == 2 && w->T == 6 && ((h->s_size == 8 && !odd) || (h->s_size == 2 && odd))) return nullptr;
+  return w;
+}
+
+// Whether some call's steps can run several to a launch.
+bool mt_possible(const flb_engine* h) { return mt_window(h, 3) || mt_window(h, kLongCall); }
 
 // Failure injection on the host: FLB_FAIL_ALLOC_AT=second in the environment
 // fails the second population buffers, as cudaMalloc does when memory runs out.
@@ -552,8 +659,8 @@ bool take_second(flb_engine* h) {
 
 // Whether this call's steps run several to a launch (h->second_mu held).  Not
 // once the caller has captured a step: the launch alternates between two buffers.
-bool mt_usable(flb_engine* h) {
-  if (h->captured || !mt_possible(h)) return false;
+bool mt_usable(flb_engine* h, uint64_t n) {
+  if (h->captured || !mt_window(h, n)) return false;
   return h->d_f2 || (h->own_second && take_second(h));
 }
 
@@ -569,10 +676,10 @@ bool caller_captures(flb_engine* h) {
   return true;
 }
 
-// One launch of at most `left` steps, the last of which writes density and
-// velocity when it is the last of `left` (wm).
-flb_status mt_launch(flb_engine* h, uint64_t left, bool wm, int& T) {
-  MtArgs a = mt_plan(h, *mt_window(h), left);
+// One launch of at most `left` steps on windows w, the last of which writes
+// density and velocity when it is the last of `left` (wm).
+flb_status mt_launch(flb_engine* h, const MtWindow& w, uint64_t left, bool wm, int& T) {
+  MtArgs a = mt_plan(h, w, left);
   refresh_params(h);
   a.dst = h->d_f2;
   a.t = (uint32_t)h->t;
@@ -590,11 +697,11 @@ flb_status mt_launch(flb_engine* h, uint64_t left, bool wm, int& T) {
 
 constexpr int kMtGraph = 8;  // launches per graph (even: the buffers end where they began)
 
-flb_status mt_capture(flb_engine* h, GraphSlot& g, int T) {
+flb_status mt_capture(flb_engine* h, GraphSlot& g, const MtWindow& w) {
   FLB_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   flb_status s = FLB_OK;
   int t = 0;
-  for (int k = 0; k < kMtGraph && s == FLB_OK; k++) s = mt_launch(h, (uint64_t)T, false, t);
+  for (int k = 0; k < kMtGraph && s == FLB_OK; k++) s = mt_launch(h, w, (uint64_t)w.T, false, t);
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
   if (s == FLB_OK && e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
@@ -612,14 +719,16 @@ flb_status mt_capture(flb_engine* h, GraphSlot& g, int T) {
 // kernels); a handle on its own is bound by the GPU, and FP16 storage needs
 // the step number in every launch.
 flb_status mt_steps(flb_engine* h, uint64_t n) {
-  const MtWindow& w = *mt_window(h);
+  const MtWindow& w = *mt_window(h, n);
   const uint64_t per = (uint64_t)kMtGraph * (uint64_t)w.T;
+  // (calls that are not long may take other windows: no graph of those)
+  const bool graphs = h->peers > 1 && h->s_size != 2 && n >= kLongCall;
   while (n > 0) {
-    if (h->peers > 1 && h->s_size != 2 && n > per) {
+    if (graphs && n > per) {
       GraphSlot& g = h->g_mt[2 * (h->d_f < h->d_f2 ? 0 : 1) + (int)(h->t & 1u)];
       if (g.exec && g.f != h->d_f) destroy_graph(g);
       if (!g.exec) {
-        const flb_status s = mt_capture(h, g, w.T);
+        const flb_status s = mt_capture(h, g, w);
         if (s != FLB_OK) return s;
       }
       FLB_CUDA(h, cudaGraphLaunch(g.exec, h->stream));
@@ -629,7 +738,7 @@ flb_status mt_steps(flb_engine* h, uint64_t n) {
       continue;
     }
     int T = 0;
-    const flb_status s = mt_launch(h, n, true, T);
+    const flb_status s = mt_launch(h, w, n, true, T);
     if (s != FLB_OK) return s;
     h->launches += 1;
     h->t += (uint64_t)T;
@@ -1135,7 +1244,7 @@ FLB_API flb_status flb_step(flb_handle h, uint64_t n) {
   flb_status s = FLB_OK;
   if (n >= 2) {
     std::lock_guard<std::mutex> lk(h->second_mu);
-    if (mt_usable(h)) {
+    if (mt_usable(h, n)) {
       s = mt_steps(h, n);
       remaining = 0;
     }
