@@ -65,3 +65,36 @@ def test_lists_match_oracle(nx, ny, prec, walls, mode):
             assert exact_equal(a, want[name]), f"t={o.t} {name}: {first_mismatch(a, want[name])}"
     s.close()
     o.close()
+
+
+# plain-fluid super-tiles (grids of more than 1,024) under the options that the
+# cases above leave out: FlowLB's free-surface rules, implicit walls, FP32 mass,
+# the reference arithmetic, the subgrid model
+@pytest.mark.parametrize("variant,kw", [
+    (O.F32_M32, dict(fs_mode=E.FS_REFERENCE, bb=E.BB_IMPLICIT, arith=E.ARITH_REFERENCE)),
+    (O.F32_M32, dict(fs_mode=E.FS_REFERENCE, bb=E.BB_IMPLICIT, arith=E.ARITH_REFERENCE, subgrid=True)),
+    (O.F32, dict(fs_mode=E.FS_CONSERVATIVE, bb=E.BB_HALFWAY, arith=E.ARITH_FUSED, subgrid=True)),
+    (O.F32_M32, dict(fs_mode=E.FS_CONSERVATIVE, bb=E.BB_IMPLICIT, arith=E.ARITH_FUSED)),
+    (O.F64, dict(fs_mode=E.FS_REFERENCE, bb=E.BB_IMPLICIT, arith=E.ARITH_REFERENCE)),
+    (O.F16S, dict(fs_mode=E.FS_REFERENCE, bb=E.BB_IMPLICIT, arith=E.ARITH_FUSED)),
+], ids=["ref-m32", "ref-m32-subgrid", "f32-subgrid", "implicit-m32", "ref-f64", "ref-f16s"])
+@pytest.mark.parametrize("nx,ny", [(2113, 266), (2176, 520)], ids=str)
+def test_plain_fluid_super_tiles_under_other_options(variant, kw, nx, ny):
+    kw = dict(kw)
+    bb, arith = kw.pop("bb"), kw.pop("arith")
+    kw.update(tau=0.56, fx=3e-4, fy=-2e-4, u_max=0.25)
+    flags = blobs(nx, ny, True)
+    prec = {O.F64: 64, O.F16S: 16}.get(variant, 32)
+    s = E.Solver(flags, free_surface=True, precision=prec, mass_precision=32 if variant == O.F32_M32 else 64,
+                 bounce_back=bb, arithmetic=arith, **kw)
+    s.set_step_mode(E.STEP_KERNELS)
+    o = O.Oracle(flags, O.OracleConfig(variant=variant, free_surface=True, bb=bb, arithmetic=arith, **kw))
+    for n in (1, 2, 5, 40):
+        s.step(n)
+        o.step(n)
+        want = oracle_fields(o, prec)
+        for name in FIELDS:
+            a = getattr(s, name)
+            assert exact_equal(a, want[name]), f"t={o.t} {name}: {first_mismatch(a, want[name])}"
+    s.close()
+    o.close()
