@@ -220,6 +220,7 @@ constexpr uint32_t kDeepTile = 0x80000000u;
 // did not stay in the SMs' instruction caches from step to step (on a tile of
 // its own the flag stencil took 5,000 cycles, nearly all of it waiting for
 // instructions).
+constexpr bool kFsOdd = false;  // the parity they are compiled for
 inline KParams as_even(const KParams& kp, uint32_t odd) {
   KParams q = kp;
   if (odd)

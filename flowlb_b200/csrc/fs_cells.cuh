@@ -12,7 +12,7 @@ namespace flb {
 // ---- FS_1: mass exchange and gas reconstruction, lbmKernel2D.cu:14-121 -----
 // flag, nbm: the cell's flag and wall mask (0 without half-way walls),
 // loaded by the caller.
-template <class S, class C, class M, bool HW, bool ODD>
+template <class S, class C, class M, bool HW>
 __device__ __forceinline__ void fs1_cell(const KParams& p, uint32_t x, uint32_t y, uint8_t flag, uint32_t nbm) {
   const uint32_t nx = p.nx, N = p.N;
   const uint32_t idx = x + y * nx;
@@ -24,8 +24,8 @@ __device__ __forceinline__ void fs1_cell(const KParams& p, uint32_t x, uint32_t 
   uint32_t nb[9];
   neighbours(x, y, nx, p.ny, nb);
   C in[9], out[9];
-  load_in<S, C, false, ODD>(p, idx, nb, 0u, in);
-  load_out<S, C, ODD>(p, idx, nb, out);
+  load_in<S, C, false, kFsOdd>(p, idx, nb, 0u, in);
+  load_out<S, C, kFsOdd>(p, idx, nb, out);
   M* Ms = static_cast<M*>(p.mass);
   const M* Ex = static_cast<const M*>(p.excess);
   const M* Ph = static_cast<const M*>(p.phi);
@@ -37,7 +37,7 @@ __device__ __forceinline__ void fs1_cell(const KParams& p, uint32_t x, uint32_t 
   const bool cons = p.fs_cons != 0;
   const uint8_t e = flag & kFGI;
   if (cons && (!(e == kFluid || e == kInterface) || (flag & kMovingWall))) return;
-  if (HW && nbm) reload_reflected<S, C, ODD>(p, idx, nb, nbm, in);
+  if (HW && nbm) reload_reflected<S, C, kFsOdd>(p, idx, nb, nbm, in);
   out[0] = in[0];
 #pragma unroll
   for (int i = 1; i < 9; i++) m += exn[i];
@@ -111,8 +111,8 @@ __device__ __forceinline__ void fs1_cell(const KParams& p, uint32_t x, uint32_t 
       const float scale = p.f16_scale;
 #pragma unroll
       for (int i = 1; i < 9; i += 2) {
-        if (nF[i + 1] == kGas) Codec<S, C>::st(slotp<S>(p, slot_a<ODD>(i)), idx, i, in[i], scale);
-        if (nF[i] == kGas) Codec<S, C>::st(slotp<S>(p, slot_b<ODD>(i)), nb[i], i + 1, in[i + 1], scale);
+        if (nF[i + 1] == kGas) Codec<S, C>::st(slotp<S>(p, slot_a<kFsOdd>(i)), idx, i, in[i], scale);
+        if (nF[i] == kGas) Codec<S, C>::st(slotp<S>(p, slot_b<kFsOdd>(i)), nb[i], i + 1, in[i + 1], scale);
       }
     }
   }
@@ -120,17 +120,17 @@ __device__ __forceinline__ void fs1_cell(const KParams& p, uint32_t x, uint32_t 
 }
 
 // The cell's flag and wall mask in one round trip, then the cell.
-template <class S, class C, class M, bool HW, bool ODD>
+template <class S, class C, class M, bool HW>
 __device__ __forceinline__ void fs1_cell(const KParams& p, uint32_t x, uint32_t y) {
   const uint32_t idx = x + y * p.nx;
   const uint8_t flag = p.flags[idx];
   const uint32_t nbm = HW ? p.nbmask[idx] : 0u;
-  fs1_cell<S, C, M, HW, ODD>(p, x, y, flag, nbm);
+  fs1_cell<S, C, M, HW>(p, x, y, flag, nbm);
 }
 
 // A cell of a deep super-tile: fluid, as all its neighbours, none of them
 // across the grid's edge or a wall.  Returns its mass, which the caller stores.
-template <class S, class C, class M, bool ODD>
+template <class S, class C, class M>
 __device__ __forceinline__ M fs1_deep_cell(const KParams& p, uint32_t idx) {
   const uint32_t nx = p.nx;
   const uint32_t nb[9] = {idx,          idx + 1u,      idx - 1u,      idx + nx,      idx - nx,
@@ -139,10 +139,10 @@ __device__ __forceinline__ M fs1_deep_cell(const KParams& p, uint32_t idx) {
   const float inv = p.f16_inv;
 #pragma unroll
   for (int i = 1; i < 9; i += 2) {
-    in[i] = Codec<S, C>::ld(slotp<S>(p, slot_a<ODD>(i)), idx, i, inv);
-    in[i + 1] = Codec<S, C>::ld(slotp<S>(p, slot_b<ODD>(i)), nb[i], i + 1, inv);
+    in[i] = Codec<S, C>::ld(slotp<S>(p, slot_a<kFsOdd>(i)), idx, i, inv);
+    in[i + 1] = Codec<S, C>::ld(slotp<S>(p, slot_b<kFsOdd>(i)), nb[i], i + 1, inv);
   }
-  load_out<S, C, ODD>(p, idx, nb, out);
+  load_out<S, C, kFsOdd>(p, idx, nb, out);
   const M* Ex = static_cast<const M*>(p.excess);
   M m = static_cast<const M*>(p.mass)[idx];
   M exn[9];
@@ -312,7 +312,7 @@ __device__ __forceinline__ void fs4_own_excess(const KParams& p, uint32_t idx, F
 // fluid or interface after the pass.  Q: the cell lies in a quiet tile (no
 // gas, interface or gas-interface cell within reach), where the byte chain
 // leaves the flag as it is and no cell turns from gas to interface.
-template <class S, class C, class M, bool ODD, int TW, bool Q>
+template <class S, class C, class M, int TW, bool Q>
 __device__ __forceinline__ bool fs234_cell(const KParams& p, const FlagMasks<TW>& sm, int gx, int gy, int lx, int ly,
                                            const Fs4Own<C, M>& own) {
   const int nx = (int)p.nx, ny = (int)p.ny;
@@ -386,7 +386,7 @@ __device__ __forceinline__ bool fs234_cell(const KParams& p, const FlagMasks<TW>
     uy = uy + rho2 * p.fy;
     limit_u(p.u_max, ux, uy);
     equilibrium(rho, ux, uy, feq);
-    store_post<S, C, ODD>(p, idx, nb, feq);
+    store_post<S, C, kFsOdd>(p, idx, nb, feq);
   }
   // FS_4 fields
   if (f3 & (kWall | kMovingWall | kInlet)) return live;
@@ -583,7 +583,7 @@ __device__ __forceinline__ void load_window(const KParams& p, int tx, int ty, in
 // tile at column xoff of a super-tile of wact x hact cells.  deep (DEEP): in,
 // whether the tile and its neighbours lie inside the grid; out, whether the
 // window is plain fluid as well, and the cells are done and the return void.
-template <class S, class C, class M, bool ODD, int TW, int CPT, bool DEEP>
+template <class S, class C, class M, int TW, int CPT, bool DEEP>
 __device__ __forceinline__ uint32_t fs234_tile(const KParams& p, int tx, int ty, int tid, FlagMasks<TW>& sm,
                                                int xoff, int wact, int hact, bool& deep) {
   constexpr int kTX = TW, kW = FlagMasks<TW>::kW, kR = FlagMasks<TW>::kR;
@@ -638,8 +638,8 @@ __device__ __forceinline__ uint32_t fs234_tile(const KParams& p, int tx, int ty,
   for (int k = 0; k < CPT; k++) {
     const int ly = ly0 + k * kRowStep, gy = ty * kTY + ly;
     if (gx < nx && gy < ny &&
-        (quiet ? fs234_cell<S, C, M, ODD, TW, true>(p, sm, gx, gy, lx, ly, own[k])
-               : fs234_cell<S, C, M, ODD, TW, false>(p, sm, gx, gy, lx, ly, own[k])))
+        (quiet ? fs234_cell<S, C, M, TW, true>(p, sm, gx, gy, lx, ly, own[k])
+               : fs234_cell<S, C, M, TW, false>(p, sm, gx, gy, lx, ly, own[k])))
       act |= activity(xoff + lx, ly, wact, hact);
   }
   return act;
@@ -734,7 +734,7 @@ __device__ __forceinline__ void append_deep(const NextLists& nl, uint32_t t) {
 // A deep super-tile (DEEP) needs neither the block's activity nor a second
 // barrier (with them: 4001x1201 68 us per step against 58.4, 8192x2048 FP32 205
 // against 197, FP16S 197 against 184).  wact_sm: one word per warp of the block.
-template <class S, class C, class M, bool ODD, int TW, int CPT, bool DEEP, bool THIN>
+template <class S, class C, class M, int TW, int CPT, bool DEEP, bool THIN>
 __device__ __forceinline__ void fs234_super_tile(const KParams& p, uint32_t t, uint32_t nsx, uint32_t* nz,
                                                  const NextLists& nl, FlagMasks<TW>& sm, uint32_t* wact_sm) {
   constexpr int kTX = TW, kWarps = TW * kTY / CPT / 32;
@@ -754,7 +754,7 @@ __device__ __forceinline__ void fs234_super_tile(const KParams& p, uint32_t t, u
     const int tx = sx * (int)(kSTW / kTX) + j;
     if (tx * kTX < (int)p.nx) {
       bool deep = sx > 0 && sy > 0 && (uint32_t)(sx + 1) * kSTW < p.nx && (uint32_t)(sy + 1) * kSTH < p.ny;
-      act |= fs234_tile<S, C, M, ODD, TW, CPT, DEEP>(p, tx, sy, tid, sm, j * kTX, wact, hact, deep);
+      act |= fs234_tile<S, C, M, TW, CPT, DEEP>(p, tx, sy, tid, sm, j * kTX, wact, hact, deep);
       if (DEEP && deep) {  // every cell is live: all activity bits
         if (tid == 0) {
           nz[t] = 0x1ffu;

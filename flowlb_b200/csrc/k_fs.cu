@@ -2,7 +2,7 @@
 // (lbmKernel2D.cu:14-121) and FS_2, FS_3, FS_4 fused into one shared-memory
 // flag-stencil kernel (lbmKernel2D.cu:124-303) that also lists the next
 // step's super-tiles.  The per-cell and per-tile code is in fs_cells.cuh.
-// Templated on the step parity.
+// Compiled for one step parity (as_even).
 #include <type_traits>
 
 #include "fs_cells.cuh"
@@ -29,7 +29,7 @@ constexpr int kFs1Block = 256;   // two cells per thread (x and x + 32 of a row)
 constexpr int kFs1Small = 512;   // one cell per thread, two blocks per SM, or one
 // lc: the next step's list lengths and marks, cleared here for this step's
 // flag pass.
-template <class S, class C, class M, bool HW, bool ODD, int BLOCK, int MB, bool DEEP>
+template <class S, class C, class M, bool HW, int BLOCK, int MB, bool DEEP>
 __global__ void __launch_bounds__(BLOCK, MB) k_fs1(const __grid_constant__ KParams p,
                                                                        const TileList tl, const ListClear lc) {
   pdl_wait();
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(BLOCK, MB) k_fs1(const __grid_constant__ KPara
       // the loads of both cells before either store
       M m[kCells];
 #pragma unroll
-      for (uint32_t k = 0; k < kCells; k++) m[k] = fs1_deep_cell<S, C, M, ODD>(p, xa + 32u * kCpr * k + y * nx);
+      for (uint32_t k = 0; k < kCells; k++) m[k] = fs1_deep_cell<S, C, M>(p, xa + 32u * kCpr * k + y * nx);
 #pragma unroll
       for (uint32_t k = 0; k < kCells; k++) static_cast<M*>(p.mass)[xa + 32u * kCpr * k + y * nx] = m[k];
       continue;
@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(BLOCK, MB) k_fs1(const __grid_constant__ KPara
       fc = p.flags[xc + y * nx];
       if (HW) mc = p.nbmask[xc + y * nx];
     }
-    if (xa < nx) fs1_cell<S, C, M, HW, ODD>(p, xa, y, fa, ma);
-    if (kCells == 2u && xc < nx) fs1_cell<S, C, M, HW, ODD>(p, xc, y, fc, mc);
+    if (xa < nx) fs1_cell<S, C, M, HW>(p, xa, y, fa, ma);
+    if (kCells == 2u && xc < nx) fs1_cell<S, C, M, HW>(p, xc, y, fc, mc);
   }
 }
 
@@ -110,7 +110,7 @@ __global__ void k_apply_recon(const __grid_constant__ KParams p, uint32_t odd) {
 // 2048x512 23.5 against 22.5), and five on grids of more than kLargeTiles
 // super-tiles, most of them plain fluid in many rounds (8192x2048 FP32 174
 // against 177, FP16S 168 against 172; 4001x1201 51.6 either way).
-template <class S, class C, class M, bool ODD, int TW, int CPT, int MB, bool THIN>
+template <class S, class C, class M, int TW, int CPT, int MB, bool THIN>
 __global__ void __launch_bounds__(TW* kTY / CPT, MB)
     k_fs234(const __grid_constant__ KParams p, const TileList tl, uint32_t* __restrict__ nz, const NextLists nl) {
   __shared__ FlagMasks<TW> sm;
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(TW* kTY / CPT, MB)
   pdl_wait();
   pdl_trigger();
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x)
-    fs234_super_tile<S, C, M, ODD, TW, CPT, (CPT > 1), THIN>(p, tile_at(tl, i), tl.nsx, nz, nl, sm, wact_sm);
+    fs234_super_tile<S, C, M, TW, CPT, (CPT > 1), THIN>(p, tile_at(tl, i), tl.nsx, nz, nl, sm, wact_sm);
 }
 
 // ---- launchers -------------------------------------------------------------------
@@ -132,8 +132,8 @@ void launch_fs1(const KParams& kp, cudaStream_t st, uint32_t odd, bool hw, const
   auto go = [&](auto block, auto mb) {
     constexpr int BLOCK = decltype(block)::value, MB = decltype(mb)::value;
     constexpr bool DEEP = BLOCK == kFs1Block;
-    if (hw) launch_pdl(k_fs1<S, C, M, true, false, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl, lc);
-    else launch_pdl(k_fs1<S, C, M, false, false, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl, lc);
+    if (hw) launch_pdl(k_fs1<S, C, M, true, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl, lc);
+    else launch_pdl(k_fs1<S, C, M, false, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl, lc);
   };
   using std::integral_constant;
   if (tl.ntiles <= kTinyTiles) go(integral_constant<int, kFs1Small>{}, integral_constant<int, 1>{});
@@ -159,8 +159,8 @@ void launch_fs234_form(const KParams& kp, cudaStream_t st, uint32_t odd, const T
   const KParams q = as_even(kp, odd);
   auto go = [&](auto thin) {
     constexpr bool THIN = decltype(thin)::value;
-    if (tl.ntiles <= kWideTiles) launch_pdl(k_fs234<S, C, M, false, TW, CPT, MB, THIN>, grid, threads, st, q, tl, nz, nl);
-    else k_fs234<S, C, M, false, TW, CPT, MB, THIN><<<grid, threads, 0, st>>>(q, tl, nz, nl);
+    if (tl.ntiles <= kWideTiles) launch_pdl(k_fs234<S, C, M, TW, CPT, MB, THIN>, grid, threads, st, q, tl, nz, nl);
+    else k_fs234<S, C, M, TW, CPT, MB, THIN><<<grid, threads, 0, st>>>(q, tl, nz, nl);
   };
   if (nl.thin) go(std::true_type{});
   else go(std::false_type{});

@@ -103,14 +103,14 @@ __device__ __forceinline__ bool fsp_step(const KParams& p, const uint32_t odd, c
   for (uint32_t i = blockIdx.x; i < nsc; i += G) {
     const uint32_t t = __ldcg(lsc + i) & ~kDeepTile;
     const uint32_t y = (t / a.nsx) * kSTH + row, x = (t % a.nsx) * kSTW + xo;
-    if (y < p.ny && x < p.nx) fs1_cell<S, C, M, HW, false>(p, x, y);
+    if (y < p.ny && x < p.nx) fs1_cell<S, C, M, HW>(p, x, y);
   }
   if (!next_barrier(a, nbar, ok)) return false;
   // stream-collide
   for (uint32_t i = blockIdx.x; i < nsc; i += G) {
     const uint32_t t = __ldcg(lsc + i) & ~kDeepTile;
     const uint32_t y = (t / a.nsx) * kSTH + row, x = (t % a.nsx) * kSTW + xo;
-    if (y < p.ny && x < p.nx) sc_cell<S, C, M, true, HW, true, false, FU>(p, x, y);
+    if (y < p.ny && x < p.nx) sc_cell<S, C, M, true, HW, true, kFsOdd, FU>(p, x, y);
   }
   if (!next_barrier(a, nbar, ok)) return false;
   // FS_2..4: flag stencil, mass / excess / fill level, activity words and the
@@ -118,7 +118,7 @@ __device__ __forceinline__ bool fsp_step(const KParams& p, const uint32_t odd, c
   const NextLists nl{a.list[odd ^ 1u][0], a.list[odd ^ 1u][1], a.lcount + 2 * (odd ^ 1u), a.lbits + (odd ^ 1u) * a.nwords,
                      a.nsx, a.nsy, a.thin};
   for (uint32_t i = blockIdx.x; i < nfs; i += G)
-    fs234_super_tile<S, C, M, false, 64, 1, false, true>(p, __ldcg(lfs + i), a.nsx, a.nz, nl, sm, wact_sm);
+    fs234_super_tile<S, C, M, 64, 1, false, true>(p, __ldcg(lfs + i), a.nsx, a.nz, nl, sm, wact_sm);
   return next_barrier(a, nbar, ok);
 }
 

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kBlock, FLB_SC_MIN_BLOCKS) k_sc_scalar(const _
 // (bound by memory) 512 x 3: 8192x2048 F32 177 us per step against 181 with 256
 // x 4 or 512 x 2, 182 with 256 x 5 and 184 with 512 x 4; 4001x1201 51.6 against
 // 52.7, 51.9, 53.3 and 53.7.
-template <class S, class C, class M, bool HW, bool ODD, bool FU, int BLOCK, int MB, bool DEEP>
+template <class S, class C, class M, bool HW, bool FU, int BLOCK, int MB, bool DEEP>
 __global__ void __launch_bounds__(BLOCK, MB) k_sc_list(const __grid_constant__ KParams p,
                                                                            const TileList tl) {
   // the list was built two kernels back (FS_1 waited for it), so it is read
@@ -82,12 +82,12 @@ __global__ void __launch_bounds__(BLOCK, MB) k_sc_list(const __grid_constant__ K
     const uint32_t xb = (t % tl.nsx) * kSTW + lane;
     if (DEEP && (e & kDeepTile)) {
 #pragma unroll 1
-      for (uint32_t j = chunk * 32u; j < kSTW; j += 32u * cpr) sc_deep_cell<S, C, M, ODD, FU>(p, xb + j, y);
+      for (uint32_t j = chunk * 32u; j < kSTW; j += 32u * cpr) sc_deep_cell<S, C, M, FU>(p, xb + j, y);
       continue;
     }
 #pragma unroll 1
     for (uint32_t j = chunk * 32u; j < kSTW; j += 32u * cpr)
-      if (xb + j < p.nx) sc_cell<S, C, M, true, HW, true, ODD, FU>(p, xb + j, y);
+      if (xb + j < p.nx) sc_cell<S, C, M, true, HW, true, kFsOdd, FU>(p, xb + j, y);
   }
 }
 
@@ -314,7 +314,7 @@ template <class S>
 __host__ __device__ constexpr int list_vec_block() {
   return (int)(kSTH * kSTW / (uint32_t)Lanes<S>::V);
 }
-template <class S, class C, class M, bool HW, bool ODD, bool FU>
+template <class S, class C, class M, bool HW, bool FU>
 __global__ void __launch_bounds__(list_vec_block<S>(), 1024 / list_vec_block<S>())
     k_sc_list_vec(const __grid_constant__ KParams p, const TileList tl) {
   constexpr uint32_t V = (uint32_t)Lanes<S>::V, LPR = kSTW / V;
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(list_vec_block<S>(), 1024 / list_vec_block<S>(
     const uint32_t t = tile_at(tl, i) & ~kDeepTile;
     const uint32_t y = (t / tl.nsx) * kSTH + row;
     const uint32_t x0 = y < p.ny ? (t % tl.nsx) * kSTW + lane * V : p.nx;
-    sc_vec_cells<S, C, M, true, HW, true, ODD, FU, LPR>(p, x0, y < p.ny ? y : 0u, lane);
+    sc_vec_cells<S, C, M, true, HW, true, kFsOdd, FU, LPR>(p, x0, y < p.ny ? y : 0u, lane);
   }
 }
 
@@ -647,15 +647,15 @@ static void launch_sc_list_f(const KParams& kp, cudaStream_t st, uint32_t odd, b
   const KParams q = as_even(kp, odd);
   if (vec) {
     constexpr int B = list_vec_block<S>();
-    if (hw) launch_pdl(k_sc_list_vec<S, C, M, true, false, FU>, grid, B, st, q, tl);
-    else launch_pdl(k_sc_list_vec<S, C, M, false, false, FU>, grid, B, st, q, tl);
+    if (hw) launch_pdl(k_sc_list_vec<S, C, M, true, FU>, grid, B, st, q, tl);
+    else launch_pdl(k_sc_list_vec<S, C, M, false, FU>, grid, B, st, q, tl);
     return;
   }
   auto go = [&](auto block, auto mb) {
     constexpr int BLOCK = decltype(block)::value, MB = decltype(mb)::value;
     constexpr bool DEEP = MB != 2;
-    if (hw) launch_pdl(k_sc_list<S, C, M, true, false, FU, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl);
-    else launch_pdl(k_sc_list<S, C, M, false, false, FU, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl);
+    if (hw) launch_pdl(k_sc_list<S, C, M, true, FU, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl);
+    else launch_pdl(k_sc_list<S, C, M, false, FU, BLOCK, MB, DEEP>, grid, BLOCK, st, q, tl);
   };
   using std::integral_constant;
   if (tl.ntiles <= kSmallTiles) go(integral_constant<int, 512>{}, integral_constant<int, 2>{});
@@ -674,8 +674,8 @@ template <class S, class C, class M>
 int sc_list_blocks_per_sm(bool vec, bool fu, uint32_t ntiles) {
   if (!vec) return ntiles <= kSmallTiles ? 2 : list_wide<C>(fu, ntiles) ? 3 : 4;  // the launch bounds
   int n = 0, m = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sc_list_vec<S, C, M, true, false, false>, list_vec_block<S>(), 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_sc_list_vec<S, C, M, true, false, true>, list_vec_block<S>(), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sc_list_vec<S, C, M, true, false>, list_vec_block<S>(), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_sc_list_vec<S, C, M, true, true>, list_vec_block<S>(), 0);
   n = n < m ? n : m;
   return n > 0 ? n : 1;
 }

@@ -228,15 +228,15 @@ __device__ __forceinline__ void sc_cell(const KParams& p, uint32_t x, uint32_t y
 
 // A cell of a deep super-tile (kDeepTile): plain fluid, its neighbours too,
 // none of them across the grid's edge.
-template <class S, class C, class M, bool ODD, bool FU>
+template <class S, class C, class M, bool FU>
 __device__ __forceinline__ void sc_deep_cell(const KParams& p, uint32_t x, uint32_t y) {
   const uint32_t nx = p.nx, idx = x + y * nx;
   const uint32_t nb[9] = {idx,          idx + 1u,      idx - 1u,      idx + nx,      idx - nx,
                           idx + nx + 1u, idx - nx - 1u, idx - nx + 1u, idx + nx - 1u};
   C f[9];
-  load_in<S, C, false, ODD>(p, idx, nb, 0u, f);
+  load_in<S, C, false, kFsOdd>(p, idx, nb, 0u, f);
   collide_cell<C, M, true, true, FU, false, S>(p, idx, x, y, kFluid, 0u, f);
-  store_post<S, C, ODD>(p, idx, nb, f);
+  store_post<S, C, kFsOdd>(p, idx, nb, f);
 }
 
 }  // namespace flb
