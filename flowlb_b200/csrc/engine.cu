@@ -1048,18 +1048,17 @@ flb_status create_handle(const flb_case_desc* desc, flb_handle* out, bool own_se
     h->use_vec = desc->kernel_variant == 2 ||
                  (desc->kernel_variant == 0 && desc->nx % V == 0 &&
                   (desc->precision == 16 || (desc->precision == 32 && fused)));
-    // free surface, the listed stream-collide: measured on a B200, the vector
-    // path is slower for FP32 (2048x512 dam break 33.3 against 29.4 us per
-    // step; 8192x2048 53.4 against 54.8 GLUPS) and faster for FP16S on large
-    // grids (8192x2048: 57.5 against 54.7 GLUPS), so it runs there, or when
-    // asked for
+    // free surface, the listed stream-collide: one cell per thread, which has a
+    // short form for super-tiles of plain fluid; the vector path when asked for.
+    // Measured on a B200, dam breaks, us per step one cell | vector: FP32 2048x512
+    // 22.0 | 28.4, 8192x2048 167 | 195, FP16S 2048x512 22.8 | 27.5, 4800x1600 74.9 |
+    // 78.0, 8192x2048 157 | 164
     const uint64_t tiles = (uint64_t)((desc->nx + kSTW - 1) / kSTW) * ((desc->ny + kSTH - 1) / kSTH);
-    h->use_vec_list = desc->kernel_variant == 2 ||
-                      (desc->kernel_variant == 0 && desc->nx % V == 0 && desc->precision == 16 && fused &&
-                       tiles > 8192u);
+    h->use_vec_list = desc->kernel_variant == 2;
     // FS_1 and the flag pass: one cell per thread on grids of up to
     // kSmallTiles super-tiles, two above (FsForm, k_fs.cu).
-    // FLB_FS_FLAG_FORM selects another flag-pass form, with the same results.
+    // FLB_FS_FLAG_FORM selects another flag-pass form, with the same results
+    // (the names of the former 128-wide tiles stand for the 64-wide ones).
     h->fs_form = tiles <= kSmallTiles ? FS_FORM_W64X1 : FS_FORM_W64X2;
     if (const char* v = std::getenv("FLB_FS_FLAG_FORM")) {
       if (!std::strcmp(v, "32")) h->fs_form = FS_FORM_W32;

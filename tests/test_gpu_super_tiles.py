@@ -98,3 +98,17 @@ def test_plain_fluid_super_tiles_under_other_options(variant, kw, nx, ny):
             assert exact_equal(a, want[name]), f"t={o.t} {name}: {first_mismatch(a, want[name])}"
     s.close()
     o.close()
+
+
+def test_fp16_listed_paths_agree_on_a_large_grid():
+    """FP16 storage above 8,192 super-tiles: the default stream-collide against the vector one."""
+    flags = blobs(4160, 1040, True)
+    kw = dict(free_surface=True, precision=16, tau=0.56, fx=3e-4, fy=-2e-4, u_max=0.25)
+    a, b = E.Solver(flags, **kw), E.Solver(flags, kernel_variant=2, **kw)
+    for n in (3, 40):
+        a.step(n)
+        b.step(n)
+        for name in FIELDS:
+            assert exact_equal(getattr(a, name), getattr(b, name)), name
+    a.close()
+    b.close()
