@@ -87,7 +87,7 @@ int fs234_blocks_per_sm(int form, uint32_t ntiles);
 constexpr uint32_t kSmallTiles = 1024, kTinyTiles = 512, kLargeTiles = 8192;
 
 // the free-surface step as one persistent cooperative kernel (k_fsp.cu):
-// a.steps steps per launch, `grid` CTAs of 1024 threads all resident at once
+// a.steps steps per launch, `grid` CTAs of 512 threads all resident at once
 template <class S, class C, class M>
 cudaError_t launch_fs_persist(const KParams& p0, const KParams& p1, const FspArgs& a, uint32_t grid, bool hw, bool fu,
                               cudaStream_t st);
