@@ -538,6 +538,9 @@ constexpr MtWindow kMtF16Odd[] = {{18000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A
                                   {300000, 148, 148, MT_ALL, FLB_MT_C(512, 0)},
                                   {270000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_ONE},
                                   {300000, 300, 300, MT_ALL, FLB_MT_C(512, 0)}};
+// ... and, with another than the fused arithmetic (TRT 401x301, us per step: 4.5 one
+// step per launch, C 5.5; calls of 20, 5.2 and 5.8; 201x200 gains), up to so many cells
+constexpr uint64_t kF16OddDear = 50000;
 // calls of fewer than kLongCall steps
 constexpr MtWindow kMtF32Short[] = {{18000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_A(384, 1)},
                                     {110000, kAnyTiles, kAnyTiles, MT_ALL, FLB_MT_B(384, 1)},
@@ -592,6 +595,8 @@ const MtWindow* mt_window(const flb_engine* h, uint64_t n) {
   if (h->fs || h->has_io || h->desc.kernel_variant != 0 || n < 2) return nullptr;
   const uint64_t cells = (uint64_t)h->N * h->peers;
   const bool narrow = h->nx < kNarrow, odd = h->nx % 4u != 0;
+  // odd FP16 rows with arithmetic that is not the fused one
+  if (h->s_size == 2 && odd && !h->fused && cells > kF16OddDear) return nullptr;
   if (n >= kLongCall || narrow || h->ny < 2u * kFewRows) {
     if (h->s_size == 8) return mt_pick(kMtF64, h, cells);
     if (h->s_size == 2) return odd && !narrow ? mt_pick(kMtF16Odd, h, cells) : mt_pick(kMtF16, h, cells);

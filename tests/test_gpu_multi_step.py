@@ -129,6 +129,7 @@ LONG += [(64, FUSED, nx, ny, True) for nx, ny in [(129, 128), (201, 200), (200, 
 LONG += [(64, FUSED, nx, ny, False) for nx, ny in [(256, 256), (50001, 3)]]
 LONG += [(16, FUSED, nx, ny, True) for nx, ny in [(129, 128), (201, 200), (200, 200), (400, 300), (301, 301), (529, 529),
                                                   (33, 3030)]]
+LONG += [(16, TRT, 201, 200, True), (16, TRT, 401, 301, False), (16, LES, 400, 300, True)]
 LONG += [(16, FUSED, nx, ny, False) for nx, ny in [(249, 249), (1549, 96), (1877, 117)]]
 
 
